@@ -61,7 +61,7 @@ XRT_HD f3 fmad(f3 a, float s, f3 b) {
 // same expression is compiled for the device and for the CPU oracle, so bend projections agree
 // bit for bit (the two platforms' acosf differ in the last place, and the bend solve amplifies
 // that).
-XRT_HD float acos_as(float x) {
+XRT_HD float acos_poly(float x) {
   float p = -0.0012624911f;
   p = fmaf(p, x, 0.0066700901f);
   p = fmaf(p, x, -0.0170881256f);
@@ -69,9 +69,9 @@ XRT_HD float acos_as(float x) {
   p = fmaf(p, x, -0.0501743046f);
   p = fmaf(p, x, 0.0889789874f);
   p = fmaf(p, x, -0.2145988016f);
-  p = fmaf(p, x, 1.5707963050f);
-  return sqrtf(1.0f - x) * p;
+  return fmaf(p, x, 1.5707963050f);
 }
+XRT_HD float acos_as(float x) { return sqrtf(1.0f - x) * acos_poly(x); }
 
 // MathFunctions::FaceNormal (src/math/MathFunctions.cu:14-20)
 XRT_HD f3 face_normal(f3 a, f3 b, f3 c) { return normalize(cross(b - a, c - a)); }

@@ -230,8 +230,8 @@ struct TiledSet {
   uint32_t max_cons = 0;                // most constraints in one tile
   uint32_t max_step = 0;                // most constraints in one local color of one tile
   uint32_t block = 512;                 // threads per tile block (256 or 512)
-  uint32_t block1 = 512;                // threads per block of the streamed (one-lane) kernels
-  uint32_t resident = 0;                // tile blocks the GPU holds at once (pair-mode bound)
+  uint32_t block1 = 512;                // threads per block of the streamed kernels
+  uint32_t resident = 0;                // tile blocks the GPU holds at once (above: streamed)
   std::vector<ColorRange> tile_colors;  // ranges of executed tiles per tile color
   std::vector<uint32_t> tile_color_cons;  // constraints per tile color (profiling units)
   DBuf<uint32_t> foot;                  // footprint vertices of every executed tile
@@ -626,7 +626,7 @@ void launch_fem(Context& c, const FrameConst& k, bool reset_lambda, int phase_st
                 int phase_bend);
 void fem_release(Context& c);
 size_t tile_smem_bytes(const TiledSet& T, size_t record_bytes);
-// the forward stretch / bend kernels (bend: lane pairs or one lane)
+// the forward stretch / bend kernels
 size_t tile_smem_fwd(const TiledSet& T, bool stretch, bool whole);
 // float4 -> packed xyz (12 B per element) and back (w set to `w`), for host copies.
 void launch_pack_xyz(const float4* in, float* out, uint32_t n, cudaStream_t s);

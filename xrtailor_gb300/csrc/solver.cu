@@ -109,7 +109,13 @@ __global__ void k_stretch(const int4* __restrict__ con, float* __restrict__ lamb
 // (TiledSet::rec: 16-bit footprint-local ids, then float2 values) into shared memory, completed
 // on mbarriers while the predecessor grid drains and the footprint is gathered.  Every wait on a
 // barrier is bounded; a copy that does not complete raises kErrBulkCopy and the block waits
-// (bounded) for its copies in flight and leaves.  NT threads per block: 512 for footprints up to
+// (bounded) for its copies in flight and leaves.  After pdl_wait one round trip brings footprint
+// and multipliers (read one after the other they took 2,000 to 2,500 cycles of a single-wave
+// launch, together 1,100 to 1,300); the rest of a launch is its chain of local colors (700 to 900
+// cycles each for bend, 450 to 550 for stretch: shared loads, the projection's dependent
+// arithmetic, a barrier) and the write-back.  Frames against two lanes per element, branching
+// roots and a late release: 64 x 64 sheet 4.48 -> 3.56 ms, 256 x 256 garment 16.5 -> 14.3 ms,
+// 768 x 701 sheet 11.4 -> 9.1 ms.  NT threads per block: 512 for footprints up to
 // 4,096 vertices, 256 (twice the resident blocks per SM) up to 2,048.
 // Stretch tiles: the record block holds one segment per local color, as for bend (16-bit ids,
 // then float2 rest length and stretch_alpha(compliance, dt), each padded to 16 bytes).  STREAM (throughput regime):
@@ -122,7 +128,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_stretch_tiles(
     float* __restrict__ lambda, float4* __restrict__ x, const uint32_t* __restrict__ foot,
     const int4* __restrict__ meta, const uint32_t* __restrict__ lofs, uint32_t tile_begin,
     uint32_t num_local, uint32_t max_foot, uint32_t max_seg16, uint32_t buf16, uint32_t max_cons,
-    uint32_t* err, float4* __restrict__ tape_x, float* __restrict__ tape_l) {
+    uint32_t* err, bool early, float4* __restrict__ tape_x, float* __restrict__ tape_l) {
   if (num_local == 0) return;  // no constraint in the schedule
   extern __shared__ float4 smem[];
   float4* sx = smem;
@@ -160,13 +166,24 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_stretch_tiles(
       if (num_local > 1) issue(1);
     }
   }
+  __syncthreads();  // the barriers' initialisation, still ahead of the predecessor's end
+  bool ok = mbar_wait_bounded(bar, 0, kBulkWaitLimit);
   pdl_wait();
+  // the first multipliers and the footprint come in one round trip
+  constexpr int kLam = 4;
+  float lam0[kLam];
+#pragma unroll
+  for (int r = 0; r < kLam; ++r)
+    lam0[r] = !RESET && threadIdx.x + r * NT < nc ? lambda[c0 + threadIdx.x + r * NT] : 0.0f;
+  tile_park<NT>(f, tile_load<NT>(f, x), sx, sf);
+#pragma unroll
+  for (int r = 0; r < kLam; ++r)
+    if (threadIdx.x + r * NT < nc) sl[threadIdx.x + r * NT] = lam0[r];
 #pragma unroll 4
-  for (uint32_t j = threadIdx.x; j < nc; j += NT) sl[j] = RESET ? 0.0f : lambda[c0 + j];
-  tile_gather<NT>(f, x, sx, sf);
-  __syncthreads();  // offsets, footprint, multipliers and the barriers' initialisation
-  auto failed = [&](bool ok, uint32_t l) {
-    if (!__syncthreads_or(!ok)) return false;
+  for (uint32_t j = threadIdx.x + kLam * NT; j < nc; j += NT)
+    sl[j] = RESET ? 0.0f : lambda[c0 + j];
+  auto failed = [&](bool fine, uint32_t l) {
+    if (!__syncthreads_or(!fine)) return false;
     if (threadIdx.x == 0) {
       raise_error(err, kErrBulkCopy);
       if (!STREAM)
@@ -178,7 +195,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_stretch_tiles(
     __syncthreads();
     return true;
   };
-  if (failed(mbar_wait_bounded(bar, 0, kBulkWaitLimit), 0)) return;
+  if (failed(ok, 0)) return;  // and the footprint and the multipliers are visible
+  if (early) pdl_release();
   uint32_t at = 0;  // whole block: the color's segment
   for (uint32_t l = 0; l < num_local; ++l) {
     const uint4* cur = STREAM ? buf + (l & 1) * max_seg16 : buf + at;
@@ -196,7 +214,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_stretch_tiles(
         tape_x[2 * slot + 1] = b;
         tape_l[slot] = lam;
       }
-      if (stretch_project_alpha(a, b, rc.x, rc.y, lam)) {
+      if (stretch_project_fast(a, b, rc.x, rc.y, lam)) {
         sx[ab.x] = a;
         sx[ab.y] = b;
         sl[cb + j] = lam;
@@ -207,12 +225,12 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_stretch_tiles(
       __syncthreads();
       continue;
     }
-    const bool ok = l + 1 >= num_local ||
-                    mbar_wait_bounded(bar + ((l + 1) & 1), ((l + 1) >> 1) & 1u, kBulkWaitLimit);
+    ok = l + 1 >= num_local ||
+         mbar_wait_bounded(bar + ((l + 1) & 1), ((l + 1) >> 1) & 1u, kBulkWaitLimit);
     if (failed(ok, l + 1)) return;
     if (threadIdx.x == 0 && l + 2 < num_local) issue(l + 2);  // into the buffer color l read
   }
-  pdl_release();  // late: the successor's blocks arrive as this one drains (measured faster)
+  if (!early) pdl_release();
   tile_scatter<NT>((uint32_t)f.m.y, x, sx, sf);
 #pragma unroll 4
   for (uint32_t j = threadIdx.x; j < nc; j += NT) lambda[c0 + j] = sl[j];
@@ -234,30 +252,22 @@ __global__ void k_bend(const int4* __restrict__ idx, const float2* __restrict__ 
   x[b.w] = a4;
 }
 
-// PAIR: two lanes per bend element (bend_project_pair), half the dependency chain per step, for
-// launches whose tiles are all resident at once (latency-bound); otherwise one lane per element
-// (fewer instructions in total, for launches with many waves of tiles).
-// Records: the tile's record block (TiledSet::rec) holds one segment per local color (16-bit
-// footprint-local ids, then float2 rest angle and bend_alpha(compliance, dt), each padded to 16
-// bytes).
-//   one lane (throughput regime): the segments stream in by local color, each bulk-copied into
-//     one of two shared-memory buffers on its own mbarrier, two colors ahead of its use; a buffer
-//     is refilled right after the barrier that closes the color that read it.  Only two colors'
-//     records occupy shared memory, so more tiles fit on an SM.
-//   lane pairs (latency regime, every tile of the launch resident): the whole block comes in one
-//     bulk copy before the first color, so no color waits on a copy.
-template <int NT, bool PAIR, bool TAPE>
+// Bend tiles: as the stretch tiles, without multipliers.  One lane per element: two lanes sharing
+// one element (half the expression each, exchanged by shuffles) were faster in single-wave launches
+// while every division and root carried a branch; with the straight-line projection one lane is
+// (a color of 64 elements alone on an SM 768 cycles against 837, of 128 elements 860 against
+// 1,043), and it issues half the warp instructions.
+template <int NT, bool STREAM, bool TAPE>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_bend_tiles(
     const uint4* __restrict__ rec, const uint32_t* __restrict__ rec_ofs, float4* __restrict__ x,
     const uint32_t* __restrict__ foot, const int4* __restrict__ meta,
     const uint32_t* __restrict__ lofs, uint32_t tile_begin, uint32_t num_local,
-    uint32_t max_foot, uint32_t max_seg16, uint32_t buf16, uint32_t* err,
+    uint32_t max_foot, uint32_t max_seg16, uint32_t buf16, uint32_t* err, bool early,
     float4* __restrict__ tape_x) {
   if (num_local == 0) return;  // no constraint in the schedule
   extern __shared__ float4 smem[];
   float4* sx = smem;
-  // buf16 uint4 of records: one lane, two buffers of max_seg16; lane pairs, the largest block
-  uint4* buf = reinterpret_cast<uint4*>(sx + max_foot);
+  uint4* buf = reinterpret_cast<uint4*>(sx + max_foot);  // buf16 uint4 (see the launcher)
   uint64_t* bar = reinterpret_cast<uint64_t*>(buf + buf16);
   uint32_t* so = reinterpret_cast<uint32_t*>(bar + 2);
   uint32_t* sf = so + num_local + 1;
@@ -278,7 +288,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bend_tiles(
     src = __ldg(&rec_ofs[t]);
     mbar_init(bar, 1);
     mbar_init(bar + 1, 1);
-    if (PAIR) {  // the whole block at once (barrier 1 completes without a copy)
+    if (!STREAM) {  // the whole block at once
       const uint32_t all = __ldg(&rec_ofs[t + 1]) - src;
       if (all)
         bulk_load_g2s(buf, rec + src, 16u * all, bar);
@@ -289,16 +299,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bend_tiles(
       if (num_local > 1) issue(1);
     }
   }
+  __syncthreads();  // the barriers' initialisation, still ahead of the predecessor's end
+  bool ok = mbar_wait_bounded(bar, 0, kBulkWaitLimit);
   pdl_wait();
   tile_gather<NT>(f, x, sx, sf);
-  __syncthreads();  // offsets, footprint and the barriers' initialisation are visible
   // a wait that runs out raises the error; the block waits (bounded) for its copies in flight
   // and leaves, the same in every thread
-  auto failed = [&](bool ok, uint32_t l) {
-    if (!__syncthreads_or(!ok)) return false;
+  auto failed = [&](bool fine, uint32_t l) {
+    if (!__syncthreads_or(!fine)) return false;
     if (threadIdx.x == 0) {
       raise_error(err, kErrBulkCopy);
-      if (PAIR)  // the one copy of the whole block
+      if (!STREAM)
         mbar_wait_bounded(bar, 0, kBulkWaitLimit);
       else
         for (uint32_t k = l; k < l + 2 && k < num_local; ++k)
@@ -307,65 +318,41 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bend_tiles(
     __syncthreads();
     return true;
   };
-  if (failed(mbar_wait_bounded(bar, 0, kBulkWaitLimit), PAIR ? num_local : 0)) return;
-  uint32_t at = 0;  // PAIR: the color's segment in the whole block
+  if (failed(ok, 0)) return;  // and the footprint is visible
+  if (early) pdl_release();
+  uint32_t at = 0;  // whole block: the color's segment
   for (uint32_t l = 0; l < num_local; ++l) {
-    const uint4* cur = PAIR ? buf + at : buf + (l & 1) * max_seg16;
+    const uint4* cur = STREAM ? buf + (l & 1) * max_seg16 : buf + at;
     const uint32_t c0 = so[l], n = so[l + 1] - c0;
     const ushort4* sid = reinterpret_cast<const ushort4*>(cur);
     const float2* st = reinterpret_cast<const float2*>(cur + (n + 1) / 2);
-    if (PAIR) {
-      // the loop trip count is warp-uniform so the pair exchanges run with full warps
-      const uint32_t lane0 = threadIdx.x & ~31u, ce = 2 * n;
-      for (uint32_t base = lane0; base < ce; base += NT) {
-        const uint32_t s = base + (threadIdx.x & 31u);
-        const bool active = s < ce;
-        const uint32_t j = active ? s >> 1 : 0;
-        const ushort4 q = sid[j];
-        const int4 b = make_int4(q.x, q.y, q.z, q.w);
-        const float2 th = st[j];
-        if (TAPE && active) {  // the adjoint's replay: each lane tapes the two inputs it owns
-          const uint32_t half = s & 1u;
-          float4* t = tape_x + 4 * ((size_t)f.m.z + c0 + j) + 2 * half;
-          t[0] = sx[half ? b.z : b.x];
-          t[1] = sx[half ? b.w : b.y];
-        }
-        bend_project_pair(sx, b, th.x, th.y, s & 1u, active);
+    for (uint32_t j = threadIdx.x; j < n; j += NT) {
+      const ushort4 b = sid[j];
+      const float2 th = st[j];
+      const float4 a1 = sx[b.x], a2 = sx[b.y], a3 = sx[b.z], a4 = sx[b.w];
+      if (TAPE) {  // the adjoint's replay: the projection's inputs by execution slot
+        float4* t = tape_x + 4 * ((size_t)f.m.z + c0 + j);
+        t[0] = a1;
+        t[1] = a2;
+        t[2] = a3;
+        t[3] = a4;
       }
-    } else {
-      for (uint32_t j = threadIdx.x; j < n; j += NT) {
-        const ushort4 b = sid[j];
-        const float2 th = st[j];
-        float4 a1 = sx[b.x], a2 = sx[b.y], a3 = sx[b.z], a4 = sx[b.w];
-        if (TAPE) {  // the adjoint's replay: the projection's inputs by execution slot
-          float4* t = tape_x + 4 * ((size_t)f.m.z + c0 + j);
-          t[0] = a1;
-          t[1] = a2;
-          t[2] = a3;
-          t[3] = a4;
-        }
-        bend_project_alpha(a1, a2, a3, a4, th.x, th.y);
-        sx[b.x] = a1;
-        sx[b.y] = a2;
-        sx[b.z] = a3;
-        sx[b.w] = a4;
-      }
+      bend_project_fast(sx, b, a1, a2, a3, a4, th.x, th.y);
     }
-    if (PAIR) {
+    if (!STREAM) {
       at += color_seg16(n, 4);
       __syncthreads();
       continue;
     }
     // the next color's records, then the barrier that closes this color
-    const bool ok = l + 1 >= num_local ||
-                    mbar_wait_bounded(bar + ((l + 1) & 1), ((l + 1) >> 1) & 1u, kBulkWaitLimit);
+    ok = l + 1 >= num_local ||
+         mbar_wait_bounded(bar + ((l + 1) & 1), ((l + 1) >> 1) & 1u, kBulkWaitLimit);
     if (failed(ok, l + 1)) return;
     if (threadIdx.x == 0 && l + 2 < num_local) issue(l + 2);  // into the buffer color l read
   }
-  pdl_release();
+  if (!early) pdl_release();
   tile_scatter<NT>((uint32_t)f.m.y, x, sx, sf);
 }
-
 
 // Free slot vertices: one launch per slot over that slot's constraint block (list order).
 __global__ void k_lra_block(const uint32_t* __restrict__ tgt, const uint32_t* __restrict__ src,
@@ -579,7 +566,7 @@ cudaError_t raise_smem(const void* kern, size_t bytes) {
 }
 
 // Every instantiation of the forward tile kernels, indexed by their template flags (reset, 512
-// threads, streamed records, tape / 512 threads, lane pairs, tape).
+// threads, streamed records, tape / 512 threads, streamed records, tape).
 using StretchTilesK = decltype(&k_stretch_tiles<false, 256, false, false>);
 using BendTilesK = decltype(&k_bend_tiles<256, false, false>);
 static const StretchTilesK kStretchTiles[16] = {
@@ -613,8 +600,8 @@ static const BendTilesK kBendTiles[8] = {
 static StretchTilesK stretch_tiles_kernel(bool reset, bool b512, bool stream, bool tape) {
   return kStretchTiles[(reset ? 8 : 0) + (b512 ? 4 : 0) + (stream ? 2 : 0) + (tape ? 1 : 0)];
 }
-static BendTilesK bend_tiles_kernel(bool b512, bool pair, bool tape) {
-  return kBendTiles[(b512 ? 4 : 0) + (pair ? 2 : 0) + (tape ? 1 : 0)];
+static BendTilesK bend_tiles_kernel(bool b512, bool stream, bool tape) {
+  return kBendTiles[(b512 ? 4 : 0) + (stream ? 2 : 0) + (tape ? 1 : 0)];
 }
 
 // The limit is a property of the kernel function on the current device, shared by every
@@ -660,11 +647,9 @@ size_t tile_smem_fwd(const TiledSet& T, bool stretch, bool whole) {
 }
 
 // Block size of a tile set: 256 threads when the footprint fits 256 x kFootPerThread and a local
-// color's elements (two lanes each for bend) fill at most one pass, else 512; and how many of its
-// bend blocks the GPU holds at once.
+// color's elements fill at most one pass, else 512; and how many of its blocks the GPU holds at once.
 cudaError_t choose_tile_block(TiledSet& T, bool bend) {
-  const uint32_t lanes = bend ? 2 * T.max_step : T.max_step;
-  T.block = (T.max_foot <= 256u * kFootPerThread && lanes <= 256) ? 256 : 512;
+  T.block = (T.max_foot <= 256u * kFootPerThread && T.max_step <= 256) ? 256 : 512;
   // streamed (throughput-regime) blocks: 256 threads whenever the footprint allows (a large color
   // takes a second pass, but twice the blocks fit on an SM)
   T.block1 = T.max_foot <= 256u * kFootPerThread ? 256 : T.block;
@@ -673,7 +658,7 @@ cudaError_t choose_tile_block(TiledSet& T, bool bend) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   const size_t smem = tile_smem_fwd(T, !bend, true);
-  const void* kern = bend ? (const void*)bend_tiles_kernel(T.block != 256, true, false)
+  const void* kern = bend ? (const void*)bend_tiles_kernel(T.block != 256, false, false)
                           : (const void*)stretch_tiles_kernel(false, T.block != 256, false, false);
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)T.block, smem);
   if (e != cudaSuccess) return e;
@@ -708,6 +693,15 @@ void launch_unpack_xyz(const float* in, float4* out, uint32_t n, float w, cudaSt
   if (n) k_unpack_xyz<<<grid_for(n), kBlock, 0, s>>>(in, out, n, w);
 }
 
+// When a tile block lets the next launch's blocks in: right after its gather when every local color
+// fits one pass of the block, else after its last color.  The tile launches follow one another, and
+// a block's prologue (metadata, footprint ids, records: 1,600 to 4,000 cycles) is then hidden behind
+// the colors of the launch before (256-vertex tiles: the 713-vertex sheet's frame 791 -> 661 us, the
+// 538 k vertex sheet's 17.0 -> 15.0 ms).  With several passes a color (1,024-vertex tiles of a
+// batch) the prologue is a small part, and blocks that arrive early fill the SMs unevenly: 29.4 ->
+// 35.4 ms.
+static bool release_early(const TiledSet& T, uint32_t block) { return T.max_step <= block; }
+
 void launch_stretch_tiles(Context& c, const FrameConst& k, ColorRange tiles, bool reset_lambda,
                           float4* tape_x, float* tape_l) {
   const uint32_t nt = tiles.end - tiles.begin;
@@ -719,23 +713,21 @@ void launch_stretch_tiles(Context& c, const FrameConst& k, ColorRange tiles, boo
   const StretchTilesK kern = stretch_tiles_kernel(reset_lambda, block != 256, stream, tape_x);
   launch_k(c.pdl, kern, nt, block, tile_smem_fwd(T, true, !stream), c.stream, T.rec.p,
            T.rec_ofs.p, c.s_lambda.p, c.x.p, T.foot.p, T.meta.p, T.lofs.p, tiles.begin,
-           T.num_local, T.max_foot, T.max_seg16, buf16, T.max_cons, c.err.p, tape_x, tape_l);
+           T.num_local, T.max_foot, T.max_seg16, buf16, T.max_cons, c.err.p,
+           release_early(T, block), tape_x, tape_l);
 }
 
 void launch_bend_tiles(Context& c, const FrameConst& k, ColorRange tiles, float4* tape_x) {
   const uint32_t nt = tiles.end - tiles.begin;
   if (nt == 0) return;
   const TiledSet& T = c.b_tiles;
-  // two lanes per element when the launch's tiles are all resident (latency-bound: halve the
-  // chain), or when every local color's lane pairs fit one pass of the block (the pairs then
-  // use lanes that would idle at the color's barrier)
-  const bool pair = nt <= T.resident || 2 * T.max_step <= T.block;
-  const uint32_t block = pair ? T.block : T.block1;
-  const BendTilesK kern = bend_tiles_kernel(block != 256, pair, tape_x);
-  const uint32_t buf16 = pair ? T.max_tile16 : 2 * T.max_seg16;  // as tile_smem_fwd sizes it
-  launch_k(c.pdl, kern, nt, block, tile_smem_fwd(T, false, pair), c.stream, T.rec.p, T.rec_ofs.p,
+  const bool stream = nt > T.resident;  // many waves of tiles: throughput regime
+  const uint32_t block = stream ? T.block1 : T.block;
+  const BendTilesK kern = bend_tiles_kernel(block != 256, stream, tape_x);
+  const uint32_t buf16 = stream ? 2 * T.max_seg16 : T.max_tile16;  // as tile_smem_fwd sizes it
+  launch_k(c.pdl, kern, nt, block, tile_smem_fwd(T, false, !stream), c.stream, T.rec.p, T.rec_ofs.p,
            c.x.p, T.foot.p, T.meta.p, T.lofs.p, tiles.begin, T.num_local, T.max_foot, T.max_seg16,
-           buf16, c.err.p, tape_x);
+           buf16, c.err.p, release_early(T, block), tape_x);
 }
 
 // LRA phase with a free slot vertex: one launch per slot block in list order.  (With every slot
