@@ -333,7 +333,7 @@ xrt_status xrt_lbvh_sizes(const xrt_lbvh* bvh, uint32_t* num_objects);
  * Same result as xrt_lbvh_build_device + xrt_lbvh_export, written to the caller's device
  * buffers: sorted_morton / sorted_objects (n), nodes (4 x (2n-1) uint32), aabbs (6 x (2n-1)
  * float), i_esc (n-1), e_esc (n).  d_pred may be NULL (= d_prims).  Asynchronous on `stream`.
- * Working memory is one fixed ~17 MiB device array per GPU (held from first use until exit):
+ * Working memory is one fixed ~11 MiB device array per GPU (held from first use until exit):
  * at most 65,536 primitives (larger n -> XRT_ERR_FACE_CAPACITY).  All calls on a GPU share that
  * array; calls whose device work overlaps race, so order them on one stream.  The first call on
  * each GPU looks up the array's device address (cudaGetSymbolAddress) with that GPU current;

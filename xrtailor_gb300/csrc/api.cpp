@@ -118,7 +118,7 @@ void record_frame(Context& c) {
   };
   const bool obstacle_updated = p.update_obstacle_animation && c.onf > 0;
   if (obstacle_updated) {  // UpdateObstacleAnimationFrame: UpdateData(tol 0) + Construct()
-    Timed t(c, kBvhBuild, 19, c.onf);
+    Timed t(c, kBvhBuild, 1 + c.bvh.build_launches(), c.onf);
     xrt::launch_prims_obstacle(c, 0.0f);
     c.bvh.construct(0.0f, c.stream, c.err.p);
   }
@@ -1728,9 +1728,7 @@ xrt_status xrt_lbvh_build_device(xrt_lbvh* b, const float* d_prims, const float*
   cudaStream_t s = stream ? (cudaStream_t)stream : b->stream;
   if (b->b.reserve(n) != cudaSuccess) return XRT_ERR_CUDA;
   b->b.n = n;
-  xrt::launch_float9_to_float4(d_prims, b->b.v.p, n, s);
-  xrt::launch_float9_to_float4(d_pred ? d_pred : d_prims, b->b.pred.p, n, s);
-  b->b.construct(scr, s, b->err.p);
+  b->b.construct(scr, s, b->err.p, d_prims, d_pred ? d_pred : d_prims);
   return cudaGetLastError() == cudaSuccess ? XRT_OK : XRT_ERR_CUDA;
 }
 
@@ -1755,8 +1753,7 @@ xrt_status xrt_lbvh_refit_device(xrt_lbvh* b, const float* d_pred, uint32_t n, v
   if (!b || !d_pred || n != b->b.n) return XRT_ERR_INVALID_ARGUMENT;
   cudaSetDevice(b->device);
   cudaStream_t s = stream ? (cudaStream_t)stream : b->stream;
-  xrt::launch_float9_to_float4(d_pred, b->b.pred.p, n, s);
-  b->b.refit_from_pred(s, b->err.p);
+  b->b.refit_from_pred(d_pred, s, b->err.p);
   return cudaGetLastError() == cudaSuccess ? XRT_OK : XRT_ERR_CUDA;
 }
 

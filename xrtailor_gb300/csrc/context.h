@@ -106,8 +106,17 @@ struct Lbvh {
   DBuf<int4> node;                 // parent, left, right, object (segment-local)
   DBuf<uint32_t> morton, index;    // sort inputs
   DBuf<uint32_t> skey, sval;       // segment pass of the sort (nseg > 1)
-  DBuf<unsigned long long> key64;
-  DBuf<uint32_t> flags;            // arrival counters of the bottom-up merge (parity)
+  DBuf<unsigned long long> slot;   // bottom-up merge: per split, the first arrival (lbvh_dev.cuh)
+  // small trees (lbvh_dev.cuh TreeRest): per block of 256 leaves the subtrees it leaves to the last
+  // block, their number, and the blocks done
+  static constexpr uint32_t kSmallBlocks = 64, kRestPerBlock = 128, kRestWords = 3;
+  static constexpr size_t rest_words(size_t n) {
+    const size_t b = (n + 255) / 256;
+    return b <= kSmallBlocks ? b * kRestPerBlock * kRestWords : 1;
+  }
+  DBuf<float4> rest;
+  DBuf<uint32_t> rest_count;
+  DBuf<uint8_t> delta;             // per sorted position: 1 + common prefix with the next key
   DBuf<int32_t> iesc, eesc;
   DBuf<float> root;                // 6 floats per segment (ordered-int encoded)
   DBuf<uint32_t> dup;              // number of equal adjacent Morton codes
@@ -121,10 +130,14 @@ struct Lbvh {
   // Uploads the table; call before reserve.
   cudaError_t set_segments(const std::vector<uint32_t>& counts, cudaStream_t s);
   cudaError_t reserve(uint32_t n_prims);
-  // BVH::Construct(scr) on v / pred already in device memory (BVH.cu:618-722), every segment.
-  void construct(float scr, cudaStream_t s, uint32_t* d_err);
-  // Leaves grow by pred (already updated), internal boxes recomputed bottom-up.
-  void refit_from_pred(cudaStream_t s, uint32_t* d_err);
+  // BVH::Construct(scr) on v / pred already in device memory (BVH.cu:618-722), every segment; or on
+  // 9 floats per primitive (single trees; p9 = pred).
+  void construct(float scr, cudaStream_t s, uint32_t* d_err, const float* v9 = nullptr,
+                 const float* p9 = nullptr);
+  // Leaves grow by pred (9 floats per primitive), internal boxes recomputed bottom-up.
+  void refit_from_pred(const float* p9, cudaStream_t s, uint32_t* d_err);
+  uint32_t build_launches() const;  // kernels of one construct()
+  bool small() const;               // few enough leaves for the small-tree kernels (lbvh_dev.cuh)
   uint32_t nseg() const { return h_seg.empty() ? 1u : (uint32_t)h_seg.size(); }
   int4 seg_one() const { return make_int4(0, (int)n, 0, 0); }
   LbvhView view() const { return LbvhView{n, pred.p, lo.p, hi.p}; }  // single-segment trees
@@ -143,7 +156,6 @@ void launch_refit_midstep(Lbvh& b, const float4* x1, const float4* n1, const int
 // Standalone query kernel: candidates of points (kind 0), segments (1), boxes (2).
 void launch_lbvh_query(const Lbvh& b, int kind, const float* d_q, uint32_t nq, uint32_t* d_counts,
                        uint32_t* d_cands, cudaStream_t s, uint32_t* d_err);
-void launch_float9_to_float4(const float* d_in, float4* d_out, uint32_t n_prims, cudaStream_t s);
 
 // ---- instances (batched form) -------------------------------------------------------------------
 // Per-instance constants.  In merged mode (the reference's one mesh of every cloth) there is one

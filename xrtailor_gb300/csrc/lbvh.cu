@@ -10,9 +10,9 @@
 // Layout: node k keeps its box and its traversal links in two float4s (32 B, one sector):
 //   lo = {lower.xyz, left child (internal) | object (leaf)}, hi = {upper.xyz, escape index}.
 // A leaf is node >= n-1.  Stackless traversal therefore reads 32 contiguous bytes per visit.
-// The hierarchy is always built on 64-bit keys (code << 32 | object): for unique codes this gives
-// exactly the tree the reference builds on 32-bit codes (every common-prefix length is decided
-// in the high word), and for duplicate codes it is the reference's own 64-bit fallback.
+// The hierarchy is that of 64-bit keys (code << 32 | object): for unique codes this is exactly the
+// tree the reference builds on 32-bit codes (every common-prefix length is decided in the high
+// word), and for duplicate codes it is the reference's own 64-bit fallback.
 #include "common.cuh"
 #include "context.h"
 #include "lbvh_dev.cuh"
@@ -36,79 +36,135 @@ __device__ __forceinline__ uint32_t morton_code(f3 p) {
   return expand_bits((uint32_t)x) * 4 + expand_bits((uint32_t)y) * 2 + expand_bits((uint32_t)z);
 }
 
-// Order-preserving float <-> uint mapping for atomic min / max of the root box.
+// Order-preserving float <-> uint mapping for atomic min / max of the root box.  A NaN (the box of a
+// triangle shrunk to a point) counts as -0.
 __device__ __forceinline__ uint32_t f2o(float f) {
   uint32_t u = __float_as_uint(f);
+  if ((u & 0x7FFFFFFFu) > 0x7F800000u) return 0x7FFFFFFFu;
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ float o2f(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-// Root boxes of every segment: 6 ordered-int extrema each.
-__global__ void k_root_init(uint32_t* root, uint32_t nseg, uint32_t* dup) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < 6 * nseg) {
-    const uint32_t k = t % 6;
-    root[t] = k < 3 ? f2o(__int_as_float(0x7f800000)) : f2o(__int_as_float((int)0xff800000));
-  }
-  if (t == 0) *dup = 0;
-}
-
-// InitAABBs_Kernel + the root reduction (thrust::reduce of Bounds::Merge), per segment.  Min /
-// max are exact, so the reduction order does not matter: warps whose lanes share one segment
-// reduce by shuffles, a warp that straddles a segment boundary commits lane by lane.
-__global__ void __launch_bounds__(kBlock) k_leaf_boxes(const float4* __restrict__ v,
-                                                       const float4* __restrict__ pred, uint32_t n,
-                                                       float scr, float4* __restrict__ leaf_lo,
-                                                       float4* __restrict__ leaf_hi,
-                                                       uint32_t* __restrict__ root, LbvhForest F) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  float lo[3] = {__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0x7f800000)};
-  float hi[3] = {-lo[0], -lo[1], -lo[2]};
-  if (i < n) {
-    f3 v1 = mk3(v[3 * i]), v2 = mk3(v[3 * i + 1]), v3 = mk3(v[3 * i + 2]);
-    f3 p1 = mk3(pred[3 * i]), p2 = mk3(pred[3 * i + 1]), p3 = mk3(pred[3 * i + 2]);
-    f3 bl = mk3(tmin(tmin(v1.x, tmin(v2.x, v3.x)), tmin(p1.x, tmin(p2.x, p3.x))),
-                tmin(tmin(v1.y, tmin(v2.y, v3.y)), tmin(p1.y, tmin(p2.y, p3.y))),
-                tmin(tmin(v1.z, tmin(v2.z, v3.z)), tmin(p1.z, tmin(p2.z, p3.z))));
-    f3 bu = mk3(tmax(tmax(v1.x, tmax(v2.x, v3.x)), tmax(p1.x, tmax(p2.x, p3.x))),
-                tmax(tmax(v1.y, tmax(v2.y, v3.y)), tmax(p1.y, tmax(p2.y, p3.y))),
-                tmax(tmax(v1.z, tmax(v2.z, v3.z)), tmax(p1.z, tmax(p2.z, p3.z))));
-    f3 center = (bl + bu) * 0.5f;
-    f3 n1 = normalize(bl - center);
-    f3 n2 = normalize(bu - center);
-    bl = bl + scr * n1;
-    bu = bu + scr * n2;
-    leaf_lo[i] = mk4(bl, 0.0f);
-    leaf_hi[i] = mk4(bu, 0.0f);
-    lo[0] = bl.x; lo[1] = bl.y; lo[2] = bl.z;
-    hi[0] = bu.x; hi[1] = bu.y; hi[2] = bu.z;
-  }
-  const uint32_t seg = i < n ? forest_find(F, i, 0) : 0xFFFFFFFFu;
-  const int lane = threadIdx.x & 31;
-  if (__match_any_sync(0xFFFFFFFFu, seg) == 0xFFFFFFFFu) {
-    if (seg == 0xFFFFFFFFu) return;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      float a = lo[k], b = hi[k];
-      for (int off = 16; off > 0; off >>= 1) {
-        a = fminf(a, __shfl_xor_sync(0xFFFFFFFFu, a, off));
-        b = fmaxf(b, __shfl_xor_sync(0xFFFFFFFFu, b, off));
-      }
-      lo[k] = a;
-      hi[k] = b;
-    }
-    if (lane != 0) return;
-  } else if (seg == 0xFFFFFFFFu) {
-    return;
-  }
-  uint32_t* r = root + 6 * (size_t)seg;
+// A primitive's six vertices (v, then pred): float4 arrays, or 9 packed floats each.
+struct Prims {
+  const float4 *v, *pred;
+  const float *v9, *p9;
+};
+struct Box {
+  f3 lo, hi;
+};
+// InitAABBs_Kernel: bounds of v and pred, corners moved outwards by scr.
+template <bool PACKED>
+__device__ __forceinline__ Box leaf_box(const Prims& P, uint32_t i, float scr) {
+  f3 v[3], q[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    atomicMin(&r[k], f2o(lo[k]));
-    atomicMax(&r[3 + k], f2o(hi[k]));
+    if (PACKED) {
+      const float *a = P.v9 + 9 * (size_t)i + 3 * k, *b = P.p9 + 9 * (size_t)i + 3 * k;
+      v[k] = mk3(a[0], a[1], a[2]);
+      q[k] = P.p9 == P.v9 ? v[k] : mk3(b[0], b[1], b[2]);
+    } else {
+      v[k] = mk3(P.v[3 * (size_t)i + k]);
+      q[k] = mk3(P.pred[3 * (size_t)i + k]);
+    }
   }
+  f3 bl = mk3(tmin(tmin(v[0].x, tmin(v[1].x, v[2].x)), tmin(q[0].x, tmin(q[1].x, q[2].x))),
+              tmin(tmin(v[0].y, tmin(v[1].y, v[2].y)), tmin(q[0].y, tmin(q[1].y, q[2].y))),
+              tmin(tmin(v[0].z, tmin(v[1].z, v[2].z)), tmin(q[0].z, tmin(q[1].z, q[2].z))));
+  f3 bu = mk3(tmax(tmax(v[0].x, tmax(v[1].x, v[2].x)), tmax(q[0].x, tmax(q[1].x, q[2].x))),
+              tmax(tmax(v[0].y, tmax(v[1].y, v[2].y)), tmax(q[0].y, tmax(q[1].y, q[2].y))),
+              tmax(tmax(v[0].z, tmax(v[1].z, v[2].z)), tmax(q[0].z, tmax(q[1].z, q[2].z))));
+  const f3 center = (bl + bu) * 0.5f;
+  const f3 n1 = normalize(bl - center);
+  const f3 n2 = normalize(bu - center);
+  return Box{bl + scr * n1, bu + scr * n2};
+}
+
+// Root boxes are kept as integers that order like the floats, the lower corners complemented, so
+// that 0 is neutral and every extremum is an atomicMax.  Extrema are exact, so the order of the
+// reduction does not matter; a warp reduces floats, everything above integers.
+// lane_extrema: one leaf's own.  In a warp of fewer than 32 leaves of a segment each lane commits, as
+// ever (a box with a NaN, of a triangle shrunk to a point, counts there and not in fminf).
+__device__ __forceinline__ void lane_extrema(const Box& b, uint32_t out[6]) {
+  out[0] = ~f2o(b.lo.x); out[1] = ~f2o(b.lo.y); out[2] = ~f2o(b.lo.z);
+  out[3] = f2o(b.hi.x); out[4] = f2o(b.hi.y); out[5] = f2o(b.hi.z);
+}
+__device__ __forceinline__ void warp_extrema(const Box& b, uint32_t out[6]) {
+  const float sum = (b.lo.x + b.lo.y) + (b.lo.z + b.hi.x) + (b.hi.y + b.hi.z);
+  if (!__any_sync(0xFFFFFFFFu, sum != sum)) {  // no NaN: the integers order alike
+    lane_extrema(b, out);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) out[k] = __reduce_max_sync(0xFFFFFFFFu, out[k]);
+    return;
+  }
+  float lo[3] = {b.lo.x, b.lo.y, b.lo.z}, hi[3] = {b.hi.x, b.hi.y, b.hi.z};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    for (int off = 16; off > 0; off >>= 1) {
+      lo[k] = fminf(lo[k], __shfl_xor_sync(0xFFFFFFFFu, lo[k], off));
+      hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xFFFFFFFFu, hi[k], off));
+    }
+    out[k] = ~f2o(lo[k]);
+    out[3 + k] = f2o(hi[k]);
+  }
+}
+__device__ __forceinline__ Box empty_box() {
+  const float inf = __int_as_float(0x7f800000);
+  return Box{mk3(inf, inf, inf), mk3(-inf, -inf, -inf)};
+}
+
+// InitAABBs_Kernel + the root reduction (thrust::reduce of Bounds::Merge), per segment; clears the
+// merge's slots.  A block whose leaves share a segment commits six extrema (one atomic each per
+// warp put 392,000 on six words for 2.09 M triangles: 269 us against 32), a warp that straddles a
+// segment boundary commits lane by lane.
+template <bool PACKED>
+__global__ void __launch_bounds__(kBlock) k_leaf_boxes(Prims P, uint32_t n, float scr,
+                                                       float4* __restrict__ leaf_lo,
+                                                       float4* __restrict__ leaf_hi,
+                                                       unsigned long long* __restrict__ slot,
+                                                       uint32_t* __restrict__ root, LbvhForest F) {
+  __shared__ uint32_t s_ext[6], s_seg;
+  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+  Box b = empty_box();
+  const uint32_t seg = i < n ? forest_find(F, i, 0) : 0xFFFFFFFFu;
+  if (threadIdx.x < 6) s_ext[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_seg = seg;
+  if (i < n) {
+    b = leaf_box<PACKED>(P, i, scr);
+    leaf_lo[i] = mk4(b.lo, 0.0f);
+    leaf_hi[i] = mk4(b.hi, 0.0f);
+    slot[i] = 0;
+  }
+  __syncthreads();
+  const bool whole = __syncthreads_and(seg == s_seg || i >= n);
+  const unsigned peers = __match_any_sync(0xFFFFFFFFu, seg);
+  if (seg != 0xFFFFFFFFu) {
+    uint32_t e[6];
+    const bool full = peers == 0xFFFFFFFFu;
+    full ? warp_extrema(b, e) : lane_extrema(b, e);
+    if (!full || (threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) atomicMax(whole ? &s_ext[k] : &root[6 * (size_t)seg + k], e[k]);
+    }
+  }
+  if (!whole) return;
+  __syncthreads();
+  if (threadIdx.x < 6) atomicMax(&root[6 * (size_t)s_seg + threadIdx.x], s_ext[threadIdx.x]);
+}
+
+__device__ __forceinline__ uint32_t morton_of(const Box& b, const uint32_t root[6]) {
+  const f3 wl = mk3(o2f(~root[0]), o2f(~root[1]), o2f(~root[2]));
+  const f3 wu = mk3(o2f(root[3]), o2f(root[4]), o2f(root[5]));
+  f3 p = 0.5f * (b.lo + b.hi);
+  p.x = p.x - wl.x;
+  p.y = p.y - wl.y;
+  p.z = p.z - wl.z;
+  p.x = p.x / (wu.x - wl.x);
+  p.y = p.y / (wu.y - wl.y);
+  p.z = p.z / (wu.z - wl.z);
+  return morton_code(p);
 }
 
 // ComputeMortons_Kernel: centre of the leaf box normalised by its segment's root box.
@@ -117,17 +173,8 @@ __global__ void k_morton(const float4* __restrict__ leaf_lo, const float4* __res
                          uint32_t* __restrict__ morton, uint32_t* __restrict__ index, LbvhForest F) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t* root = root_all + 6 * (size_t)forest_find(F, i, 0);
-  const f3 wl = mk3(o2f(root[0]), o2f(root[1]), o2f(root[2]));
-  const f3 wu = mk3(o2f(root[3]), o2f(root[4]), o2f(root[5]));
-  f3 p = 0.5f * (mk3(leaf_lo[i]) + mk3(leaf_hi[i]));
-  p.x = p.x - wl.x;
-  p.y = p.y - wl.y;
-  p.z = p.z - wl.z;
-  p.x = p.x / (wu.x - wl.x);
-  p.y = p.y / (wu.y - wl.y);
-  p.z = p.z / (wu.z - wl.z);
-  morton[i] = morton_code(p);
+  morton[i] = morton_of(Box{mk3(leaf_lo[i]), mk3(leaf_hi[i])},
+                        root_all + 6 * (size_t)forest_find(F, i, 0));
   index[i] = i;
 }
 
@@ -150,164 +197,236 @@ __global__ void k_seg_gather(const uint32_t* __restrict__ perm, const uint32_t* 
   i_out[p] = i_in[q];
 }
 
-// ConstructLeafNodes_Kernel + leaf boxes in sorted order + 64-bit keys + uniqueness count.
-// Objects and keys use segment-local primitive ids.
-__global__ void k_leaves(const uint32_t* __restrict__ smorton, const uint32_t* __restrict__ sindex,
-                         const float4* __restrict__ leaf_lo, const float4* __restrict__ leaf_hi,
-                         uint32_t n, float4* __restrict__ lo, float4* __restrict__ hi,
-                         int4* __restrict__ node, unsigned long long* __restrict__ key64,
-                         uint32_t* __restrict__ dup, LbvhForest F) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int4 r = forest_rec(F, forest_find(F, i, 0));
-  const uint32_t li = i - (uint32_t)r.x;
-  const uint32_t gobj = sindex[i];
-  const uint32_t obj = gobj - (uint32_t)r.x;
-  const uint32_t k = (uint32_t)r.z + (uint32_t)r.y - 1 + li;
-  const float4 a = leaf_lo[gobj], b = leaf_hi[gobj];
-  lo[k] = make_float4(a.x, a.y, a.z, __int_as_float((int)obj));
-  hi[k] = make_float4(b.x, b.y, b.z, __int_as_float(-1));
-  node[k] = make_int4(-1, -1, -1, (int)obj);
-  const uint32_t m = smorton[i];
-  key64[i] = ((unsigned long long)m << 32) | obj;
-  if (li > 0 && smorton[i - 1] == m) atomicAdd(dup, 1u);
+// Common prefix of sorted positions i and i + 1 of one segment plus one, on keys (code << 32 |
+// segment-local object); objects of a segment compare as their global ids do.
+__device__ __forceinline__ uint8_t prefix_of(uint32_t m0, uint32_t o0, uint32_t m1, uint32_t o1,
+                                             uint32_t base) {
+  return (uint8_t)(m0 != m1 ? 1 + __clz(m0 ^ m1) : 33 + __clz((o0 - base) ^ (o1 - base)));
 }
-
-__device__ __forceinline__ int cub64(unsigned long long a, unsigned long long b) {
-  return __clzll((long long)(a ^ b));
-}
-
-// ConstructInternalNodes64Bits_Kernel with determine_range / find_split, one thread per internal
-// node of the forest, on its segment's keys with local ids.
-__global__ void k_internal(const unsigned long long* __restrict__ code_all, uint32_t n_internal,
-                           float4* __restrict__ lo_all, int4* __restrict__ node_all, LbvhForest F) {
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n_internal) return;
-  const int4 r = forest_rec(F, forest_find(F, g, 3));
-  const uint32_t idx = g - (uint32_t)r.w;
-  const uint32_t n = (uint32_t)r.y;
-  const unsigned long long* __restrict__ code = code_all + r.x;
-  float4* __restrict__ lo = lo_all + r.z;
-  int4* __restrict__ node = node_all + r.z;
-  uint32_t first, last;
-  if (idx == 0) {
-    first = 0;
-    last = n - 1;
-  } else {
-    const unsigned long long self = code[idx];
-    const int L = cub64(self, code[idx - 1]);
-    const int R = cub64(self, code[idx + 1]);
-    const int d = (R > L) ? 1 : -1;
-    const int dmin = min(L, R);
-    int lmax = 2;
-    int delta = -1;
-    int it = (int)idx + d * lmax;
-    if (0 <= it && it < (int)n) delta = cub64(self, code[it]);
-    while (delta > dmin) {
-      lmax <<= 1;
-      it = (int)idx + d * lmax;
-      delta = -1;
-      if (0 <= it && it < (int)n) delta = cub64(self, code[it]);
+__global__ void __launch_bounds__(kBlock) k_deltas(const uint32_t* __restrict__ smorton,
+                                                   const uint32_t* __restrict__ sindex, uint32_t n,
+                                                   uint8_t* __restrict__ delta,
+                                                   uint32_t* __restrict__ dup, LbvhForest F) {
+  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+  bool same = false;
+  if (i < n) {
+    const int4 r = forest_rec(F, forest_find(F, i, 0));
+    uint8_t d = 0;
+    if (i + 1 < (uint32_t)(r.x + r.y)) {
+      const uint32_t m0 = smorton[i], m1 = smorton[i + 1];
+      d = prefix_of(m0, sindex[i], m1, sindex[i + 1], (uint32_t)r.x);
+      same = m0 == m1;
     }
-    int l = 0;
-    for (int t = lmax >> 1; t > 0; t >>= 1) {
-      it = (int)idx + (l + t) * d;
-      delta = -1;
-      if (0 <= it && it < (int)n) delta = cub64(self, code[it]);
-      if (delta > dmin) l += t;
-    }
-    uint32_t j = (uint32_t)((int)idx + l * d);
-    first = d < 0 ? j : idx;
-    last = d < 0 ? idx : j;
+    delta[i] = d;
   }
-  uint32_t gamma;
-  {
-    const unsigned long long fc = code[first], lc = code[last];
-    if (fc == lc) {
-      gamma = (first + last) >> 1;
-    } else {
-      const int dn = cub64(fc, lc);
-      int split = (int)first;
-      int stride = (int)(last - first);
-      do {
-        stride = (stride + 1) >> 1;
-        const int middle = split + stride;
-        if (middle < (int)last && cub64(fc, code[middle]) > dn) split = middle;
-      } while (stride > 1);
-      gamma = (uint32_t)split;
+  const unsigned eq = __ballot_sync(0xFFFFFFFFu, same);
+  if (eq && (threadIdx.x & 31) == 0) atomicAdd(dup, (uint32_t)__popc(eq));
+}
+
+// ConstructLeafNodes_Kernel, ConstructInternalNodes64Bits_Kernel, the escape tables and the boxes
+// in one bottom-up walk (tree_up).
+template <bool SMALL>
+__global__ void __launch_bounds__(kTreeBlock) k_tree(const uint32_t* __restrict__ sindex,
+                                                     const float4* __restrict__ leaf_lo,
+                                                     const float4* __restrict__ leaf_hi, uint32_t n,
+                                                     TreeMem t, uint32_t* err) {
+  extern __shared__ float4 smem[];
+  const uint32_t i = blockIdx.x * kTreeBlock + threadIdx.x;
+  f3 bl = mk3(0, 0, 0), bu = bl;
+  uint32_t obj = 0;
+  if (i < n) {
+    obj = sindex[i];
+    bl = mk3(leaf_lo[obj]);
+    bu = mk3(leaf_hi[obj]);
+    obj -= (uint32_t)forest_rec(t.F, forest_find(t.F, i, 0)).x;
+  }
+  if (SMALL)
+    small_tree<true>(t, *reinterpret_cast<SmallShared*>(smem), i, i < n, obj, bl, bu, err);
+  else
+    tree_up<true>(t, *reinterpret_cast<TreeShared*>(smem), i, i < n, obj, bl, bu, err);
+}
+
+// ---- small single trees -------------------------------------------------------------------------
+// Everything ahead of k_tree in one launch of one cluster: leaf boxes, root box, Morton codes, the
+// stable radix sort (four 8-bit digits) and the neighbors' prefixes.  As 17 launches of a few blocks
+// it was bound by the latency of launches and single-block scans (13,776 triangles: 78 us of kernels,
+// now 28; with k_tree a whole build 129 -> 50 us); the phases here are a cluster barrier apart
+// (0.2 us) and the digit counts cross the blocks through distributed shared memory.
+// A warp owns R x 32 consecutive primitives (sorted positions in later passes), so ranking them round
+// by round with one running count per warp and digit is stable; the blocks share the warps evenly.
+// A lane finds its equals by eight ballots (match.any took 3,000 cycles a pass with 64 groups on an
+// SM).
+constexpr int kSortCtas = 8;  // the portable cluster size
+constexpr int kSortThreads = 1024;
+constexpr int kSortWarps = kSortThreads / 32;
+static_assert(kSmallMax <= 2 * kSortCtas * kSortThreads, "two primitives a thread");
+
+struct SortShared {
+  uint32_t cnt[kSortWarps][256];  // per warp: digit counts, then offsets
+  uint32_t total[kSortCtas][256], base[256], part[4][256], warp[8];  // total: every block's
+  uint32_t ext[6], exts[kSortCtas][6], root[6];
+};
+
+template <bool PACKED, int R>
+__global__ void __cluster_dims__(kSortCtas, 1, 1) __launch_bounds__(kSortThreads)
+    k_small_sort(Prims P, uint32_t n, float scr, float4* __restrict__ leaf_lo,
+                 float4* __restrict__ leaf_hi, uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp,
+                 uint32_t* vals_tmp, uint8_t* __restrict__ delta, uint32_t* __restrict__ dup,
+                 TreeMem t) {
+  __shared__ SortShared sh;
+  uint32_t(*s_cnt)[256] = sh.cnt;
+  uint32_t(*s_part)[256] = sh.part;
+  uint32_t(*s_total)[256] = sh.total;
+  uint32_t *s_base = sh.base, *s_warp = sh.warp, *s_ext = sh.ext, *s_root = sh.root;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, cta = blockIdx.x;
+  // warps with primitives per block
+  const uint32_t warps = ((n + 32 * R - 1) / (32 * R) + kSortCtas - 1) / kSortCtas;
+  const uint32_t first = warp < warps ? (cta * warps + warp) * (R * 32) + lane : n + lane;
+  if (tid < 6) s_ext[tid] = 0;
+  if (cta == 0 && tid == 0) *dup = *t.ticket = 0;
+  cluster_sync();  // every block runs before the first write into another's memory
+  Box box[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint32_t i = first + 32 * r;
+    box[r] = empty_box();
+    if (i < n) {
+      box[r] = leaf_box<PACKED>(P, i, scr);
+      leaf_lo[i] = mk4(box[r].lo, 0.0f);
+      leaf_hi[i] = mk4(box[r].hi, 0.0f);
+      t.slot[i] = 0;
+    }
+    if (i - lane >= n) continue;  // uniform in the warp
+    const bool full = i - lane + 32 <= n;
+    uint32_t e[6];
+    full ? warp_extrema(box[r], e) : lane_extrema(box[r], e);
+    if (full ? lane == 0 : i < n) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) atomicMax(&s_ext[k], e[k]);
     }
   }
-  uint32_t left = gamma, right = gamma + 1;
-  if (min(first, last) == gamma) left += n - 1;
-  if (max(first, last) == gamma + 1) right += n - 1;
-  node[idx].y = (int)left;
-  node[idx].z = (int)right;
-  node[idx].w = -1;
-  node[left].x = (int)idx;
-  node[right].x = (int)idx;
-  if (idx == 0) node[0].x = -1;
-  lo[idx].w = __int_as_float((int)left);
-}
-
-// Bottom-up merge from the leaf at sorted position i (forest-wide), within its segment.
-__device__ __forceinline__ void merge_from_leaf(const LbvhForest& F, uint32_t i, float4* lo,
-                                                float4* hi, const int4* node, uint32_t* flags,
-                                                uint32_t* err) {
-  const int4 r = forest_rec(F, forest_find(F, i, 0));
-  const uint32_t n = (uint32_t)r.y;
-  if (n < 2) return;
-  lbvh_merge_upwards(n - 1 + (i - (uint32_t)r.x), n, lo + r.z, hi + r.z, node + r.z, flags + r.w,
-                     err);
-}
-
-__global__ void k_build_internal_boxes(uint32_t n, float4* lo, float4* hi, const int4* node,
-                                       uint32_t* flags, uint32_t* err, LbvhForest F) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  merge_from_leaf(F, i, lo, hi, node, flags, err);
-}
-
-// BuildInternal/ExternalEscapeIndexTable_Kernel, stored in hi.w and in the export tables (internal
-// nodes at internal_base, leaves at prim_base of their segment), one thread per forest node.
-__global__ void k_escape(uint32_t n_nodes, const int4* __restrict__ node_all,
-                         float4* __restrict__ hi_all, int32_t* __restrict__ iesc,
-                         int32_t* __restrict__ eesc, uint32_t* err, LbvhForest F) {
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n_nodes) return;
-  const int4 r = forest_rec(F, forest_find(F, g, 2));
-  const uint32_t n = (uint32_t)r.y;
-  const uint32_t k = g - (uint32_t)r.z;
-  const int4* __restrict__ node = node_all + r.z;
-  const int parent = node[k].x;
-  int esc = -1;
-  if (parent >= 0) {
-    if ((int)k == node[parent].y) {
-      esc = node[parent].z;
-    } else {
-      int cur = parent;
-      uint32_t steps = 0;
-      while (true) {
-        if (++steps > n) {
-          raise_error(err, kErrTreeWalk);
-          break;
-        }
-        const int up = node[cur].x;
-        if (up < 0) {
-          esc = -1;
-          break;
-        }
-        if (cur == node[up].z) {
-          cur = up;
-        } else {
-          esc = node[up].z;
-          break;
-        }
+  __syncthreads();
+  if (tid < 6 * kSortCtas) st_cluster(&sh.exts[cta][tid % 6], tid / 6, s_ext[tid % 6]);
+  cluster_sync();
+  if (tid < 6) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int c = 0; c < kSortCtas; ++c) m = max(m, sh.exts[c][tid]);
+    s_root[tid] = m;
+  }
+  __syncthreads();
+  uint32_t key[R], val[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint32_t i = first + 32 * r;
+    key[r] = i < n ? morton_of(box[r], s_root) : 0u;
+    val[r] = i;
+  }
+#pragma unroll 1
+  for (int pass = 0; pass < 4; ++pass) {
+    const int shift = 8 * pass;
+    uint32_t* ko = pass & 1 ? keys : keys_tmp;
+    uint32_t* vo = pass & 1 ? vals : vals_tmp;
+    if (pass) {
+      const uint32_t* ki = pass & 1 ? keys_tmp : keys;
+      const uint32_t* vi = pass & 1 ? vals_tmp : vals;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t i = first + 32 * r;
+        key[r] = i < n ? __ldcg(&ki[i]) : 0u;
+        val[r] = i < n ? __ldcg(&vi[i]) : 0u;
       }
     }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s_cnt[warp][lane + 32 * k] = 0;
+    __syncwarp();
+    uint32_t rank[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool has = first + 32 * r < n;
+      const uint32_t d = (key[r] >> shift) & 0xFFu;
+      unsigned peers = __ballot_sync(0xFFFFFFFFu, has);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const unsigned one = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? one : ~one;
+      }
+      const uint32_t before = has ? s_cnt[warp][d] : 0u;
+      rank[r] = before + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+      __syncwarp();
+      if (has && (int)lane == __ffs(peers) - 1) s_cnt[warp][d] = before + (uint32_t)__popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    {  // offsets of the warps inside the block: a quarter of the warps per thread, then the quarters
+      const uint32_t d = tid & 255u, q = tid >> 8;
+      uint32_t run = 0;
+#pragma unroll
+      for (int w = 0; w < kSortWarps / 4; ++w) {
+        const uint32_t c = s_cnt[q * (kSortWarps / 4) + w][d];
+        s_cnt[q * (kSortWarps / 4) + w][d] = run;
+        run += c;
+      }
+      s_part[q][d] = run;
+      __syncthreads();
+      // every block gets every block's totals (two blocks per quarter), so that the sums after the
+      // barrier read its own memory
+      const uint32_t sum = s_part[0][d] + s_part[1][d] + s_part[2][d] + s_part[3][d];
+      st_cluster(&s_total[cta][d], 2 * q, sum);
+      st_cluster(&s_total[cta][d], 2 * q + 1, sum);
+    }
+    cluster_sync();
+    if (tid < 256) {  // the digit's first position: smaller digits, then earlier blocks
+      uint32_t all = 0, mine = 0;
+#pragma unroll
+      for (uint32_t c = 0; c < kSortCtas; ++c) {
+        const uint32_t v = s_total[c][tid];
+        mine += c < cta ? v : 0u;
+        all += v;
+      }
+      uint32_t x = all;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+        if (lane >= (uint32_t)off) x += y;
+      }
+      if (lane == 31) s_warp[warp] = x;
+      s_base[tid] = x - all + mine;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t before = 0;
+      for (uint32_t w = 0; w < warp; ++w) before += s_warp[w];
+      s_base[tid] += before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (first + 32 * r >= n) continue;
+      const uint32_t d = (key[r] >> shift) & 0xFFu, q = warp / (kSortWarps / 4);
+      uint32_t dst = s_base[d] + s_cnt[warp][d] + rank[r];
+      for (uint32_t k = 0; k < q; ++k) dst += s_part[k][d];
+      __stcg(&ko[dst], key[r]);
+      __stcg(&vo[dst], val[r]);
+    }
+    cluster_sync();  // the pass's output is visible, and every block has read the totals
   }
-  hi_all[g].w = __int_as_float(esc);
-  if (k + 1 < n) iesc[r.w + k] = esc;
-  else eesc[r.x + k - (n - 1)] = esc;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint32_t i = first + 32 * r;
+    bool same = false;
+    if (i < n) {
+      uint8_t d = 0;
+      if (i + 1 < n) {
+        const uint32_t m0 = __ldcg(&keys[i]), m1 = __ldcg(&keys[i + 1]);
+        d = prefix_of(m0, __ldcg(&vals[i]), m1, __ldcg(&vals[i + 1]), 0);
+        same = m0 == m1;
+      }
+      delta[i] = d;
+    }
+    const unsigned eq = __ballot_sync(0xFFFFFFFFu, same);
+    if (eq && lane == 0) atomicAdd(dup, (uint32_t)__popc(eq));
+  }
 }
 
 __global__ void k_prims_mesh(const float4* __restrict__ x, const float4* __restrict__ nrm,
@@ -342,58 +461,37 @@ __global__ void k_prims_ccd(const float4* __restrict__ x, const float4* __restri
   }
 }
 
-// Forest node of the leaf at sorted position i, and its global primitive (from the leaf's
-// local object).
-__device__ __forceinline__ uint32_t leaf_node_of(const LbvhForest& F, uint32_t i, uint32_t& base) {
-  const int4 r = forest_rec(F, forest_find(F, i, 0));
-  base = (uint32_t)r.x;
-  return (uint32_t)r.z + (uint32_t)r.y - 1 + (i - (uint32_t)r.x);
-}
-
-// RefitExternalNodeMidstep_Kernel + AssignAABBCAS_Kernel, fused.
-__global__ void k_refit_midstep(uint32_t n, const float4* __restrict__ x1,
-                                const float4* __restrict__ n1, const int4* __restrict__ tri,
-                                float tol, float4* pred, float4* lo, float4* hi, const int4* node,
-                                uint32_t* flags, uint32_t* err, LbvhForest F) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t base;
-  const uint32_t k = leaf_node_of(F, i, base);
-  float4 l = lo[k], h = hi[k];
-  const uint32_t obj = base + (uint32_t)__float_as_int(l.w);
-  const int4 t = tri[obj];
-  const int id[3] = {t.x, t.y, t.z};
+// RefitExternalNodeMidstep_Kernel: the leaf at node k grows by its triangle's midstep vertices moved
+// along their normals, which become its primitive.
+struct GrowMidstep {
+  const float4 *x1, *n1;
+  const int4* tri;
+  float tol;
+  float4* pred;
+  __device__ __forceinline__ void operator()(uint32_t prim, f3& l, f3& h) const {
+    const int4 v = tri[prim];
+    const int id[3] = {v.x, v.y, v.z};
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const f3 q = mk3(x1[id[c]]) + tol * mk3(n1[id[c]]);
-    pred[3 * obj + c] = mk4(q, 0.0f);
-    l.x = tmin(l.x, q.x); l.y = tmin(l.y, q.y); l.z = tmin(l.z, q.z);
-    h.x = tmax(h.x, q.x); h.y = tmax(h.y, q.y); h.z = tmax(h.z, q.z);
+    for (int c = 0; c < 3; ++c) {
+      const f3 q = mk3(x1[id[c]]) + tol * mk3(n1[id[c]]);
+      pred[3 * (size_t)prim + c] = mk4(q, 0.0f);
+      l = mk3(tmin(l.x, q.x), tmin(l.y, q.y), tmin(l.z, q.z));
+      h = mk3(tmax(h.x, q.x), tmax(h.y, q.y), tmax(h.z, q.z));
+    }
   }
-  __stcg(&lo[k], l);
-  __stcg(&hi[k], h);
-  merge_from_leaf(F, i, lo, hi, node, flags, err);
-}
-
-// RefitExternalNode_Kernel(predicted) with per-primitive pred already in place.
-__global__ void k_refit_pred(uint32_t n, const float4* __restrict__ pred, float4* lo, float4* hi,
-                             const int4* node, uint32_t* flags, uint32_t* err, LbvhForest F) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t base;
-  const uint32_t k = leaf_node_of(F, i, base);
-  float4 l = lo[k], h = hi[k];
-  const uint32_t obj = base + (uint32_t)__float_as_int(l.w);
+};
+// RefitExternalNode_Kernel(predicted), 9 floats per primitive.
+struct GrowPred {
+  const float* p9;
+  __device__ __forceinline__ void operator()(uint32_t prim, f3& l, f3& h) const {
+    const float* q = p9 + 9 * (size_t)prim;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const f3 q = mk3(pred[3 * obj + c]);
-    l.x = tmin(l.x, q.x); l.y = tmin(l.y, q.y); l.z = tmin(l.z, q.z);
-    h.x = tmax(h.x, q.x); h.y = tmax(h.y, q.y); h.z = tmax(h.z, q.z);
+    for (int c = 0; c < 3; ++c) {
+      l = mk3(tmin(l.x, q[3 * c]), tmin(l.y, q[3 * c + 1]), tmin(l.z, q[3 * c + 2]));
+      h = mk3(tmax(h.x, q[3 * c]), tmax(h.y, q[3 * c + 1]), tmax(h.z, q[3 * c + 2]));
+    }
   }
-  __stcg(&lo[k], l);
-  __stcg(&hi[k], h);
-  merge_from_leaf(F, i, lo, hi, node, flags, err);
-}
+};
 
 }  // namespace
 
@@ -422,13 +520,6 @@ __global__ void k_query(LbvhView b, const float* __restrict__ q, uint32_t nq,
   else
     lbvh_traverse(b, [&](float4 l, float4 h) { return overlap_box(l, h, a, c); }, visit, err);
   counts[i] = found;
-}
-
-__global__ void k_float9_to_float4(const float* __restrict__ in, float4* __restrict__ out,
-                                   uint32_t n_points) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_points) return;
-  out[i] = make_float4(in[3 * i], in[3 * i + 1], in[3 * i + 2], 0.0f);
 }
 
 }  // namespace
@@ -465,8 +556,10 @@ cudaError_t Lbvh::reserve(uint32_t np) {
   if (e == cudaSuccess) e = node.reserve(nn);
   if (e == cudaSuccess) e = morton.reserve(np);
   if (e == cudaSuccess) e = index.reserve(np);
-  if (e == cudaSuccess) e = key64.reserve(np);
-  if (e == cudaSuccess) e = flags.reserve(np);
+  if (e == cudaSuccess) e = slot.reserve(np);
+  if (e == cudaSuccess) e = rest.reserve(rest_words(np));
+  if (e == cudaSuccess) e = rest_count.reserve(kSmallBlocks + 1);
+  if (e == cudaSuccess) e = delta.reserve(np);
   if (e == cudaSuccess) e = iesc.reserve(np);
   if (e == cudaSuccess) e = eesc.reserve(np);
   if (e == cudaSuccess) e = root.reserve(6 * (size_t)nseg());
@@ -475,7 +568,16 @@ cudaError_t Lbvh::reserve(uint32_t np) {
   return e;
 }
 
-void Lbvh::construct(float scr, cudaStream_t s, uint32_t* d_err) {
+template <bool PACKED>
+static void launch_small_sort(const Lbvh& b, const Prims& P, float scr, cudaStream_t s) {
+  auto k = b.n <= kSmallMax / 2 ? k_small_sort<PACKED, 1> : k_small_sort<PACKED, 2>;
+  k<<<kSortCtas, kSortThreads, 0, s>>>(P, b.n, scr, b.leaf_lo.p, b.leaf_hi.p, b.morton.p,
+                                       b.index.p, b.sorter.keys_tmp.p, b.sorter.vals_tmp.p,
+                                       b.delta.p, b.dup.p, tree_mem(b));
+}
+
+void Lbvh::construct(float scr, cudaStream_t s, uint32_t* d_err, const float* v9,
+                     const float* p9) {
   active = n > 0;
   if (n == 0) return;
   const LbvhForest F = forest();
@@ -491,45 +593,65 @@ void Lbvh::construct(float scr, cudaStream_t s, uint32_t* d_err) {
       internal += r.y ? (uint32_t)r.y - 1 : 0;
     }
   }
-  uint32_t* rootu = reinterpret_cast<uint32_t*>(root.p);
-  k_root_init<<<grid_for(6 * S), kBlock, 0, s>>>(rootu, S, dup.p);
-  k_leaf_boxes<<<grid_for(n), kBlock, 0, s>>>(v.p, pred.p, n, scr, leaf_lo.p, leaf_hi.p, rootu, F);
-  k_morton<<<grid_for(n), kBlock, 0, s>>>(leaf_lo.p, leaf_hi.p, rootu, n, morton.p, index.p, F);
-  // Morton codes have 30 bits: four 8-bit passes leave the result in (morton, index)
-  sorter.sort(morton.p, index.p, n, 30, s, &sorted_morton, &sorted_index);
-  if (S > 1) {
-    int bits = 0;
-    while ((1u << bits) < S) ++bits;
-    k_seg_keys<<<grid_for(n), kBlock, 0, s>>>(sorted_index, n, skey.p, sval.p, F);
-    uint32_t *k2 = nullptr, *perm = nullptr;
-    sorter.sort(skey.p, sval.p, n, bits, s, &k2, &perm);
-    // gather into whichever key / value pair the segment pass's result does not occupy
-    const bool in_own = perm == sval.p;
-    uint32_t* m_out = in_own ? sorter.keys_tmp.p : skey.p;
-    uint32_t* i_out = in_own ? sorter.vals_tmp.p : sval.p;
-    k_seg_gather<<<grid_for(n), kBlock, 0, s>>>(perm, sorted_morton, sorted_index, n, m_out, i_out);
-    sorted_morton = m_out;
-    sorted_index = i_out;
+  const Prims P{v.p, pred.p, v9, p9};
+  if (small()) {
+    v9 ? launch_small_sort<true>(*this, P, scr, s) : launch_small_sort<false>(*this, P, scr, s);
+    sorted_morton = morton.p;
+    sorted_index = index.p;
+  } else {
+    uint32_t* rootu = reinterpret_cast<uint32_t*>(root.p);
+    cudaMemsetAsync(rootu, 0, sizeof(uint32_t) * 6 * S, s);
+    cudaMemsetAsync(dup.p, 0, sizeof(uint32_t), s);
+    auto boxes = v9 ? k_leaf_boxes<true> : k_leaf_boxes<false>;
+    boxes<<<grid_for(n), kBlock, 0, s>>>(P, n, scr, leaf_lo.p, leaf_hi.p, slot.p, rootu, F);
+    k_morton<<<grid_for(n), kBlock, 0, s>>>(leaf_lo.p, leaf_hi.p, rootu, n, morton.p, index.p, F);
+    // Morton codes have 30 bits: four 8-bit passes leave the result in (morton, index)
+    sorter.sort(morton.p, index.p, n, 30, s, &sorted_morton, &sorted_index);
+    if (S > 1) {
+      int bits = 0;
+      while ((1u << bits) < S) ++bits;
+      k_seg_keys<<<grid_for(n), kBlock, 0, s>>>(sorted_index, n, skey.p, sval.p, F);
+      uint32_t *k2 = nullptr, *perm = nullptr;
+      sorter.sort(skey.p, sval.p, n, bits, s, &k2, &perm);
+      // gather into whichever key / value pair the segment pass's result does not occupy
+      const bool in_own = perm == sval.p;
+      uint32_t* m_out = in_own ? sorter.keys_tmp.p : skey.p;
+      uint32_t* i_out = in_own ? sorter.vals_tmp.p : sval.p;
+      k_seg_gather<<<grid_for(n), kBlock, 0, s>>>(perm, sorted_morton, sorted_index, n, m_out, i_out);
+      sorted_morton = m_out;
+      sorted_index = i_out;
+    }
+    k_deltas<<<grid_for(n), kBlock, 0, s>>>(sorted_morton, sorted_index, n, delta.p, dup.p, F);
   }
-  k_leaves<<<grid_for(n), kBlock, 0, s>>>(sorted_morton, sorted_index, leaf_lo.p, leaf_hi.p, n, lo.p,
-                                          hi.p, node.p, key64.p, dup.p, F);
-  if (internal > 0) {
-    k_internal<<<grid_for(internal), kBlock, 0, s>>>(key64.p, internal, lo.p, node.p, F);
-    cudaMemsetAsync(flags.p, 0, sizeof(uint32_t) * internal, s);
-    k_build_internal_boxes<<<grid_for(n), kBlock, 0, s>>>(n, lo.p, hi.p, node.p, flags.p, d_err, F);
-  }
-  k_escape<<<grid_for(nodes), kBlock, 0, s>>>(nodes, node.p, hi.p, iesc.p, eesc.p, d_err, F);
+  auto tree = small() ? k_tree<true> : k_tree<false>;
+  const size_t smem = small() ? sizeof(SmallShared) : sizeof(TreeShared);
+  if (raise_smem((const void*)tree, smem) != cudaSuccess) return;
+  tree<<<grid_for(n, kTreeBlock), kTreeBlock, smem, s>>>(sorted_index, leaf_lo.p, leaf_hi.p, n,
+                                                         tree_mem(*this), d_err);
 }
 
-void Lbvh::refit_from_pred(cudaStream_t s, uint32_t* d_err) {
+static_assert(kSmallMax == Lbvh::kSmallBlocks * kTreeBlock &&
+                  sizeof(TreeRest) == 16 * Lbvh::kRestWords && kRestPerBlock == Lbvh::kRestPerBlock,
+              "small trees: blocks and lists as reserved");
+bool Lbvh::small() const { return nseg() == 1 && n <= kSmallMax; }
+
+uint32_t Lbvh::build_launches() const {
+  if (small()) return 2;
+  const uint32_t pass = RadixSort::hist_entries(n) <= RadixSort::kSingleBlockScan ? 3 : 5;
+  uint32_t bits = 0;
+  while ((1u << bits) < nseg()) ++bits;
+  return 4 + pass * (4 + (bits + 7) / 8) + (nseg() > 1 ? 2 : 0);
+}
+
+void Lbvh::refit_from_pred(const float* p9, cudaStream_t s, uint32_t* d_err) {
   if (!active) return;
-  k_refit_pred<<<grid_for(n), kBlock, 0, s>>>(n, pred.p, lo.p, hi.p, node.p, flags.p, d_err,
-                                              forest());
+  launch_refit(*this, GrowPred{p9}, s, d_err);
 }
 
 void Lbvh::release() {
   v.release(); pred.release(); leaf_lo.release(); leaf_hi.release(); lo.release(); hi.release();
-  node.release(); morton.release(); index.release(); key64.release(); flags.release();
+  node.release(); morton.release(); index.release(); slot.release(); delta.release();
+  rest.release(); rest_count.release();
   iesc.release(); eesc.release(); root.release(); dup.release(); skey.release(); sval.release();
   seg.release();
   sorter.keys_tmp.release(); sorter.vals_tmp.release(); sorter.hist.release(); sorter.sums.release();
@@ -550,8 +672,7 @@ void launch_prims_ccd(Lbvh& b, const float4* x, const float4* x0, const float4* 
 void launch_refit_midstep(Lbvh& b, const float4* x1, const float4* n1, const int4* tri, float tol,
                           cudaStream_t s, uint32_t* d_err) {
   if (!b.active) return;
-  k_refit_midstep<<<grid_for(b.n), kBlock, 0, s>>>(b.n, x1, n1, tri, tol, b.pred.p, b.lo.p, b.hi.p,
-                                                   b.node.p, b.flags.p, d_err, b.forest());
+  launch_refit(b, GrowMidstep{x1, n1, tri, tol, b.pred.p}, s, d_err);
 }
 
 void launch_lbvh_query(const Lbvh& b, int kind, const float* d_q, uint32_t nq, uint32_t* d_counts,
@@ -563,11 +684,6 @@ void launch_lbvh_query(const Lbvh& b, int kind, const float* d_q, uint32_t nq, u
     k_query<1><<<grid_for(nq), kBlock, 0, s>>>(b.view(), d_q, nq, d_counts, d_cands, d_err);
   else
     k_query<2><<<grid_for(nq), kBlock, 0, s>>>(b.view(), d_q, nq, d_counts, d_cands, d_err);
-}
-
-void launch_float9_to_float4(const float* d_in, float4* d_out, uint32_t n_prims, cudaStream_t s) {
-  if (n_prims == 0) return;
-  k_float9_to_float4<<<grid_for(3 * n_prims), kBlock, 0, s>>>(d_in, d_out, 3 * n_prims);
 }
 
 }  // namespace xrt

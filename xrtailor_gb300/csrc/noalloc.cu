@@ -10,7 +10,7 @@
 // Limits and sharing:
 //   - at most kNoAllocMaxPrims (65,536) primitives per call; larger inputs are rejected with
 //     XRT_ERR_FACE_CAPACITY before any work is queued;
-//   - the scratch array is about 17 MiB per GPU.  It exists on every GPU that loads this
+//   - the scratch array is about 11 MiB per GPU.  It exists on every GPU that loads this
 //     library, from the first use on that GPU until the process exits;
 //   - every call on a GPU uses the same array, which keeps the last call's contents.  Each call
 //     clears what it relies on being zero.  Calls whose device work overlaps in time (different
@@ -32,15 +32,13 @@ constexpr uint32_t kNoAllocMaxPrims = 65536;
 constexpr size_t al(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct Layout {
-  size_t v, pred, leaf_lo, leaf_hi, lo, hi, node, morton, index, keys_tmp, vals_tmp, hist, sums,
-      key64, flags, iesc, eesc, root, dup, err, total;
+  size_t leaf_lo, leaf_hi, lo, hi, node, morton, index, keys_tmp, vals_tmp, hist, sums, slot,
+      delta, rest, rest_count, iesc, eesc, root, dup, err, total;
 };
 
 constexpr Layout make_layout(size_t n) {
   Layout L{};
   size_t o = 0;
-  L.v = o;        o += al(3 * n * 16);
-  L.pred = o;     o += al(3 * n * 16);
   L.leaf_lo = o;  o += al(n * 16);
   L.leaf_hi = o;  o += al(n * 16);
   L.lo = o;       o += al(2 * n * 16);
@@ -52,8 +50,10 @@ constexpr Layout make_layout(size_t n) {
   L.vals_tmp = o; o += al(n * 4);
   L.hist = o;     o += al(RadixSort::hist_entries(n) * 4);
   L.sums = o;     o += al(RadixSort::sums_entries(n) * 4);
-  L.key64 = o;    o += al(n * 8);
-  L.flags = o;    o += al(n * 4);
+  L.slot = o;     o += al(n * 8);
+  L.delta = o;    o += al(n);
+  L.rest = o;     o += al(Lbvh::rest_words(Lbvh::kSmallBlocks * 256) * 16);
+  L.rest_count = o; o += al((Lbvh::kSmallBlocks + 1) * 4);
   L.iesc = o;     o += al(n * 4);
   L.eesc = o;     o += al(n * 4);
   L.root = o;     o += al(6 * 4);
@@ -96,14 +96,29 @@ cudaError_t scratch_address(unsigned char** out) {
   return cudaSuccess;
 }
 
-__global__ void k_export_boxes(const float4* __restrict__ lo, const float4* __restrict__ hi,
-                               uint32_t nn, float* __restrict__ out) {
+// The caller's six arrays in one launch, in 4-byte stores (they need no more alignment than that).
+__global__ void k_export_tree(const uint32_t* __restrict__ morton, const uint32_t* __restrict__ index,
+                              const int4* __restrict__ node, const float4* __restrict__ lo,
+                              const float4* __restrict__ hi, const int32_t* __restrict__ iesc,
+                              const int32_t* __restrict__ eesc, uint32_t n,
+                              uint32_t* __restrict__ o_morton, uint32_t* __restrict__ o_objects,
+                              uint32_t* __restrict__ o_nodes, float* __restrict__ o_boxes,
+                              int32_t* __restrict__ o_iesc, int32_t* __restrict__ o_eesc) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nn) return;
+  if (k >= 2 * n - 1) return;
+  const int4 v = node[k];
   const float4 a = lo[k], b = hi[k];
-  float* r = out + 6 * (size_t)k;
+  uint32_t* w = o_nodes + 4 * (size_t)k;
+  w[0] = (uint32_t)v.x; w[1] = (uint32_t)v.y; w[2] = (uint32_t)v.z; w[3] = (uint32_t)v.w;
+  float* r = o_boxes + 6 * (size_t)k;
   r[0] = a.x; r[1] = a.y; r[2] = a.z;
   r[3] = b.x; r[4] = b.y; r[5] = b.z;
+  if (k + 1 < n) o_iesc[k] = iesc[k];
+  if (k < n) {
+    o_morton[k] = morton[k];
+    o_objects[k] = index[k];
+    o_eesc[k] = eesc[k];
+  }
 }
 
 template <typename T>
@@ -131,8 +146,6 @@ extern "C" xrt_status xrt_lbvh_build_noalloc(const float* d_prims, const float* 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t N = kNoAllocMaxPrims;
   Lbvh b;
-  point_at(b.v, base, kLayout.v, 3 * N);
-  point_at(b.pred, base, kLayout.pred, 3 * N);
   point_at(b.leaf_lo, base, kLayout.leaf_lo, N);
   point_at(b.leaf_hi, base, kLayout.leaf_hi, N);
   point_at(b.lo, base, kLayout.lo, 2 * N);
@@ -144,33 +157,22 @@ extern "C" xrt_status xrt_lbvh_build_noalloc(const float* d_prims, const float* 
   point_at(b.sorter.vals_tmp, base, kLayout.vals_tmp, N);
   point_at(b.sorter.hist, base, kLayout.hist, RadixSort::hist_entries(N));
   point_at(b.sorter.sums, base, kLayout.sums, RadixSort::sums_entries(N));
-  point_at(b.key64, base, kLayout.key64, N);
-  point_at(b.flags, base, kLayout.flags, N);
+  point_at(b.slot, base, kLayout.slot, N);
+  point_at(b.delta, base, kLayout.delta, N);
+  point_at(b.rest, base, kLayout.rest, Lbvh::rest_words(Lbvh::kSmallBlocks * 256));
+  point_at(b.rest_count, base, kLayout.rest_count, Lbvh::kSmallBlocks + 1);
   point_at(b.iesc, base, kLayout.iesc, N);
   point_at(b.eesc, base, kLayout.eesc, N);
   point_at(b.root, base, kLayout.root, 6);
   point_at(b.dup, base, kLayout.dup, 1);
   uint32_t* err = reinterpret_cast<uint32_t*>(base + kLayout.err);
   b.n = n;
-  // Zero what the build relies on: the error word here; the arrival counters and the root box
-  // are reset inside construct() (cudaMemsetAsync / k_root_init).  Every other array is fully
-  // overwritten before it is read.
+  // Zero what the build relies on: the error word here; the merge's slots, the root box and the
+  // duplicate count inside construct().  Every other array is fully overwritten before it is read.
   if (cudaMemsetAsync(err, 0, sizeof(uint32_t), s) != cudaSuccess) return XRT_ERR_CUDA;
-  launch_float9_to_float4(d_prims, b.v.p, n, s);
-  launch_float9_to_float4(d_pred ? d_pred : d_prims, b.pred.p, n, s);
-  b.construct(scr, s, err);
-  const size_t nn = 2 * (size_t)n - 1;
-  cudaError_t e = cudaMemcpyAsync(d_sorted_morton, b.sorted_morton, 4 * (size_t)n,
-                                  cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_sorted_objects, b.sorted_index, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_nodes, b.node.p, 16 * nn, cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess && n > 1)
-    e = cudaMemcpyAsync(d_iesc, b.iesc.p, 4 * ((size_t)n - 1), cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_eesc, b.eesc.p, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
-  if (e != cudaSuccess) return XRT_ERR_CUDA;
-  k_export_boxes<<<grid_for((uint32_t)nn), kBlock, 0, s>>>(b.lo.p, b.hi.p, (uint32_t)nn, d_aabbs);
+  b.construct(scr, s, err, d_prims, d_pred ? d_pred : d_prims);
+  k_export_tree<<<grid_for(2 * n - 1), kBlock, 0, s>>>(
+      b.sorted_morton, b.sorted_index, b.node.p, b.lo.p, b.hi.p, b.iesc.p, b.eesc.p, n,
+      d_sorted_morton, d_sorted_objects, d_nodes, d_aabbs, d_iesc, d_eesc);
   return cudaGetLastError() == cudaSuccess ? XRT_OK : XRT_ERR_CUDA;
 }

@@ -212,33 +212,29 @@ __device__ __forceinline__ void accumulate(const PNodes& u, const Impulse& imp, 
 // Update(faces, ccd = true): pred = x of the face, leaf box grows by the x / x0 bounds, then the
 // bottom-up merge.  `node_base` offsets face node ids (0 for the cloth, V for the obstacle) into
 // the positions arrays passed here.
-__global__ void k_update_ccd(uint32_t n, const float4* __restrict__ x, const float4* __restrict__ x0,
-                             const int4* __restrict__ tri, float4* pred, float4* lo, float4* hi,
-                             const int4* node, uint32_t* flags, uint32_t* err) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t k = n - 1 + i;
-  float4 l = lo[k], hh = hi[k];
-  const uint32_t obj = (uint32_t)__float_as_int(l.w);
-  const int4 t = tri[obj];
-  const int id[3] = {t.x, t.y, t.z};
-  float fl[3] = {__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0x7f800000)};
-  float fh[3] = {-fl[0], -fl[1], -fl[2]};
+struct GrowCcd {
+  const float4 *x, *x0;
+  const int4* tri;
+  float4* pred;
+  __device__ __forceinline__ void operator()(uint32_t prim, f3& l, f3& h) const {
+    const int4 v = tri[prim];
+    const int id[3] = {v.x, v.y, v.z};
+    float fl[3] = {__int_as_float(0x7f800000), __int_as_float(0x7f800000),
+                   __int_as_float(0x7f800000)};
+    float fh[3] = {-fl[0], -fl[1], -fl[2]};
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const f3 a = mk3(x[id[c]]), b = mk3(x0[id[c]]);
-    pred[3 * obj + c] = mk4(a, 0.0f);
-    fl[0] = tmin(fl[0], a.x); fl[1] = tmin(fl[1], a.y); fl[2] = tmin(fl[2], a.z);
-    fh[0] = tmax(fh[0], a.x); fh[1] = tmax(fh[1], a.y); fh[2] = tmax(fh[2], a.z);
-    fl[0] = tmin(fl[0], b.x); fl[1] = tmin(fl[1], b.y); fl[2] = tmin(fl[2], b.z);
-    fh[0] = tmax(fh[0], b.x); fh[1] = tmax(fh[1], b.y); fh[2] = tmax(fh[2], b.z);
+    for (int c = 0; c < 3; ++c) {
+      const f3 a = mk3(x[id[c]]), b = mk3(x0[id[c]]);
+      pred[3 * (size_t)prim + c] = mk4(a, 0.0f);
+      fl[0] = tmin(fl[0], a.x); fl[1] = tmin(fl[1], a.y); fl[2] = tmin(fl[2], a.z);
+      fh[0] = tmax(fh[0], a.x); fh[1] = tmax(fh[1], a.y); fh[2] = tmax(fh[2], a.z);
+      fl[0] = tmin(fl[0], b.x); fl[1] = tmin(fl[1], b.y); fl[2] = tmin(fl[2], b.z);
+      fh[0] = tmax(fh[0], b.x); fh[1] = tmax(fh[1], b.y); fh[2] = tmax(fh[2], b.z);
+    }
+    l = mk3(tmin(l.x, fl[0]), tmin(l.y, fl[1]), tmin(l.z, fl[2]));
+    h = mk3(tmax(h.x, fh[0]), tmax(h.y, fh[1]), tmax(h.z, fh[2]));
   }
-  l.x = tmin(l.x, fl[0]); l.y = tmin(l.y, fl[1]); l.z = tmin(l.z, fl[2]);
-  hh.x = tmax(hh.x, fh[0]); hh.y = tmax(hh.y, fh[1]); hh.z = tmax(hh.z, fh[2]);
-  __stcg(&lo[k], l);
-  __stcg(&hi[k], hh);
-  lbvh_merge_upwards(k, n, lo, hi, node, flags, err);
-}
+};
 
 // CountPairs_Kernel (no candidate limit): queries are the leaves of `lhs` in sorted order.
 template <bool FILL>
@@ -721,8 +717,7 @@ void launch_cloth_bvh_build(Context& c) {
 void launch_update_ccd(Lbvh& b, const float4* x, const float4* x0, const int4* tri, cudaStream_t s,
                        uint32_t* err) {
   if (!b.active) return;
-  k_update_ccd<<<grid_for(b.n), kBlock, 0, s>>>(b.n, x, x0, tri, b.pred.p, b.lo.p, b.hi.p, b.node.p,
-                                                b.flags.p, err);
+  launch_refit(b, GrowCcd{x, x0, tri, b.pred.p}, s, err);
 }
 
 // UpdatePairs: cloth BVH Update(ccd), then cloth x obstacle and cloth x cloth pairs.
