@@ -57,45 +57,52 @@ __device__ __forceinline__ float comp4(float4 v, int j) {
   return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));
 }
 
-// Two sums of one value per thread each, every thread getting both; the tree256 order, taken
-// separately by every group of 256 threads of the block.  ws: 18 floats per group; callers
+// N sums of one value per thread each, every thread getting all; the tree256 order, taken
+// separately by every group of 256 threads of the block.  ws: 9 N floats per group; callers
 // alternate two ws buffers, so a call needs no barrier after its reads.
-__device__ __forceinline__ void tree256_2(float& a, float& b, float* wsg) {
+template <int N>
+__device__ __forceinline__ void tree256_n(float (&v)[N], float* wsg) {
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7;
-  float* ws = wsg + 18 * (threadIdx.x >> 8);
+  float* ws = wsg + 9 * N * (threadIdx.x >> 8);
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const float oa = __shfl_down_sync(0xFFFFFFFFu, a, d);
-    const float ob = __shfl_down_sync(0xFFFFFFFFu, b, d);
-    if ((lane & (2 * d - 1)) == 0) {
-      a += oa;
-      b += ob;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const float o = __shfl_down_sync(0xFFFFFFFFu, v[q], d);
+      if ((lane & (2 * d - 1)) == 0) v[q] += o;
     }
   }
   if (lane == 0) {
-    ws[warp] = a;
-    ws[9 + warp] = b;
+#pragma unroll
+    for (int q = 0; q < N; ++q) ws[9 * q + warp] = v[q];
   }
   __syncthreads();
   if (warp == 0) {
-    float u = lane < 8 ? ws[lane] : 0.0f, w = lane < 8 ? ws[9 + lane] : 0.0f;
+    float u[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) u[q] = lane < 8 ? ws[9 * q + lane] : 0.0f;
 #pragma unroll
     for (int d = 1; d < 8; d <<= 1) {
-      const float ou = __shfl_down_sync(0xFFFFFFFFu, u, d);
-      const float ow = __shfl_down_sync(0xFFFFFFFFu, w, d);
-      if ((lane & (2 * d - 1)) == 0) {
-        u += ou;
-        w += ow;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const float o = __shfl_down_sync(0xFFFFFFFFu, u[q], d);
+        if ((lane & (2 * d - 1)) == 0) u[q] += o;
       }
     }
     if (lane == 0) {
-      ws[8] = u;
-      ws[17] = w;
+#pragma unroll
+      for (int q = 0; q < N; ++q) ws[9 * q + 8] = u[q];
     }
   }
   __syncthreads();
-  a = ws[8];
-  b = ws[17];
+#pragma unroll
+  for (int q = 0; q < N; ++q) v[q] = ws[9 * q + 8];
+}
+__device__ __forceinline__ void tree256_2(float& a, float& b, float* wsg) {
+  float v[2] = {a, b};
+  tree256_n(v, wsg);
+  a = v[0];
+  b = v[1];
 }
 
 // Sum of one value per thread of a 256-thread block in the order of the reference's stride tree:
@@ -358,6 +365,175 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kZT * G)
   if (tid == 0 && rank == 0) a.conv[zi] = conv_it;
 }
 
+// The same solve of a zone with at most one node and one impact per thread of its cluster (all but
+// zones of more than 16,384): the same operations on every value and the same sums, with what a
+// thread owns in registers.  Bounded by latency, a chain of cluster barriers, sums and gathers
+// through the L2, so each is done as seldom as the algorithm allows:
+//   - an impact's weights, normal and fixed nodes' terms are read once; a constraint then gathers
+//     only the optimized nodes' positions;
+//   - the constraint at an accepted position is kept for the multiplier and for the next
+//     iteration's coefficients, which evaluated it again;
+//   - sums that are needed at the same point share one tree (4 per iteration + 2 per search step,
+//     where 5 + 3 were), and the next position needs no copy and no barrier of its own;
+//   - a block's chunk sums go to every block's shared memory ahead of the barrier, so the totals
+//     read their own.
+template <int C, int G>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kZT * G)
+    k_zone_solve_one(ZoneArgs a, const int32_t* __restrict__ zid) {
+  constexpr int kSums = C * G;                 // chunks of the cluster
+  __shared__ float part[3][4][kSums];          // [buffer set][quantity][chunk], every block's copy
+  __shared__ float wsb[2][36 * G];
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x;
+  const int grp = tid >> 8, lt = tid & (kZT - 1);  // group, thread of the group
+  const int rank = (int)cl.block_rank(), ch = rank * G + grp;
+  const int zi = zid[blockIdx.x / C];
+  const int4 z = a.zone[zi];
+  const int eb = z.x, ni = z.y - z.x, nb = z.z, nn = z.w - z.z;
+  const int nce = (ni + kZT - 1) / kZT, ncn = (nn + kZT - 1) / kZT;
+  const int e = ch * kZT + lt;  // this thread's impact and node
+  const bool has_e = e < ni, has_k = e < nn;
+  int wsp = 0;
+  // this chunk's sums of `v` to every block, then (after the barrier) the totals over the chunks:
+  // quantity q over nc[q] chunks, the same tree in every group
+  auto publish = [&](int set, const float* v, int n) {
+    for (int t = lt; t < C * n; t += kZT) {
+      const int q = t % n;
+      float x = v[0];
+      if (q == 1) x = v[1];
+      if (n > 2 && q == 2) x = v[2];
+      if (n > 2 && q == 3) x = v[3];
+      cl.map_shared_rank(&part[set][q][ch], t / n)[0] = x;
+    }
+  };
+  float w[4] = {0, 0, 0, 0}, term[4] = {0, 0, 0, 0}, lam = 0.0f, c = 0.0f;
+  int loc[4] = {-1, -1, -1, -1};
+  f3 n = mk3(0, 0, 0);
+  if (has_e) {
+    const uint32_t id = a.zimp[eb + e];
+    const float4 sw = a.sw[id];
+    n = mk3(a.sn[id]);
+    const uint4 nd = a.snodes[id];
+    const uint32_t nds[4] = {nd.x, nd.y, nd.z, nd.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w[j] = comp4(sw, j);
+      loc[j] = a.zloc[4 * (eb + e) + j];
+      if (loc[j] < 0) term[j] = w[j] * dot(n, pos_of(a, nds[j]));
+    }
+  }
+  auto constraint = [&]() {  // constraint_at the positions in Xt
+    float v = -a.thickness;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v += loc[j] > -1 ? w[j] * dot(n, mk3(__ldcg(&a.Xt[loc[j]]))) : term[j];
+    return v;
+  };
+  f3 x = mk3(0, 0, 0), xt = x, x1 = x, g = x;
+  float m = 0.0f;
+  uint32_t s0 = 0, s1 = 0;
+  const int idx = nb + e;
+  if (has_k) {  // Initialize_Kernel
+    const uint32_t v = a.znode[idx];
+    x = xt = pos_of(a, v);
+    x1 = x1_of(a, v);
+    m = mass_of(a, v);
+    s0 = a.gptr[idx];
+    s1 = a.gptr[idx + 1];
+    __stcg(&a.Xt[idx], mk4(x, 0.0f));
+  }
+  zone_sync<C>(cl);
+  const float inv = *a.inv_avg;
+  if (has_e) c = constraint();
+  float s = kStepCoeff * (float)nn;  // InitStepLength_Kernel
+  int conv_it = kMaxOptIters, set = 0;
+  for (int it = 0; it < kMaxOptIters; ++it) {
+    float v[4] = {0, 0, 0, 0};  // C2, L2, G2, O
+    // coefficients min(c + lambda / mu, 0)
+    if (has_e) {
+      const float q = tmin(c + lam / kMu, 0.0f);
+      __stcg(&a.cc[eb + e], q);
+      v[0] = q * q;
+      v[1] = lam * lam;
+    }
+    zone_sync<C>(cl);
+    // gradient at X: inv * m * (x - x1) + sum of mu * coefficient * w_j * n (slot order)
+    if (has_k) {
+      g = (inv * m) * (x - x1);
+      f3 acc = mk3(0.0f, 0.0f, 0.0f);
+      for (uint32_t q = s0; q < s1; ++q) {
+        const uint32_t slot = a.gslot[q];
+        const int ei = (int)(slot >> 2), j = (int)(slot & 3u);
+        const uint32_t id = a.zimp[ei];
+        const f3 t = ((kMu * __ldcg(&a.cc[ei])) * comp4(a.sw[id], j)) * mk3(a.sn[id]);
+        acc = q == s0 ? t : acc + t;
+      }
+      g = g + acc;
+      v[2] = dot(g, g);
+      const f3 d = x - x1;
+      v[3] = m * dot(d, d);
+    }
+    tree256_n(v, wsb[wsp]);
+    wsp ^= 1;
+    publish(0, v, 4);
+    zone_sync<C>(cl);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = lt < (q < 2 ? nce : ncn) ? part[0][q][lt] : 0.0f;
+    tree256_n(v, wsb[wsp]);
+    wsp ^= 1;
+    const float C2 = v[0], L2 = v[1], G2 = v[2], O = v[3];
+    const float f = (0.5f * inv) * O + (0.5f * kMu) * C2 - (0.5f * L2) / kMu;
+    s = s / 0.7f;  // PreconditionStepLength_Kernel
+    float ct = 0.0f;
+    for (int ls = 0;; ++ls) {
+      s = s * 0.7f;  // AdjustStepLength_Kernel
+      float u[2] = {0, 0};  // Ot, C2t
+      if (has_k) {  // NextX_Kernel + CollisionObjective_Kernel
+        xt = x - s * g;
+        __stcg(&a.Xt[idx], mk4(xt, 0.0f));
+        const f3 d = xt - x1;
+        u[0] = m * dot(d, d);
+      }
+      zone_sync<C>(cl);  // publishes Xt
+      if (has_e) {
+        ct = constraint();
+        const float q = tmin(ct + lam / kMu, 0.0f);
+        u[1] = q * q;
+      }
+      tree256_n(u, wsb[wsp]);
+      wsp ^= 1;
+      set = set == 1 ? 2 : 1;  // written again only after a later barrier
+      publish(set, u, 2);
+      zone_sync<C>(cl);
+      u[0] = lt < ncn ? part[set][0][lt] : 0.0f;
+      u[1] = lt < nce ? part[set][1][lt] : 0.0f;
+      tree256_n(u, wsb[wsp]);
+      wsp ^= 1;
+      // BacktrackingLineSearchAdvanced_Kernel (ParallelImpactZoneOptimizer.cu:413-497)
+      const float ft = (0.5f * inv) * u[0] + (0.5f * kMu) * u[1] - (0.5f * L2) / kMu;
+      if (s < kEpsS || ft < f - (kAlpha * s) * G2 || tabs(f - ft) < kEpsF) break;
+      if (ls + 1 >= kMaxLineSearch) {  // only a non-finite objective gets here
+        if (tid == 0 && rank == 0) raise_error(a.err, kErrLineSearch);
+        s = 0.0f;
+        break;
+      }
+    }
+    if (s < kEpsS) {  // UpdateConvergency_Kernel
+      conv_it = it;
+      break;
+    }
+    x = xt;  // current_X = next_X
+    c = ct;
+    lam = tmin(lam + kMu * c, 0.0f);  // UpdateMultiplier_Kernel
+  }
+  if (has_k) {
+    __stcg(&a.X[idx], mk4(x, 0.0f));
+    __stcg(&a.Xt[idx], mk4(xt, 0.0f));
+  }
+  zone_sync<C>(cl);  // no block leaves while another writes to its shared memory
+  if (tid == 0 && rank == 0) a.conv[zi] = conv_it;
+}
+
 // 16-block clusters need the non-portable cluster size opt-in; they are used once the device
 // reports that it can hold one (else zones stay on 8-block clusters).
 // Which 16-block clusters the current device holds: bit 0 with blocks of 256 threads, bit 1 with
@@ -382,8 +558,11 @@ int wide_clusters() {
       int n = 0;
       return cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0;
     };
-    if (fits((const void*)k_zone_solve<kZoneClusterWide, 1>, kZT)) st |= 1;
-    if (fits((const void*)k_zone_solve<kZoneClusterWide, kWideGroups>, kWideGroups * kZT))
+    if (fits((const void*)k_zone_solve<kZoneClusterWide, 1>, kZT) &&
+        fits((const void*)k_zone_solve_one<kZoneClusterWide, 1>, kZT))
+      st |= 1;
+    if (fits((const void*)k_zone_solve<kZoneClusterWide, kWideGroups>, kWideGroups * kZT) &&
+        fits((const void*)k_zone_solve_one<kZoneClusterWide, kWideGroups>, kWideGroups * kZT))
       st |= 2;
     (void)cudaGetLastError();  // a refused opt-in is not an error of the step
     state[dev] = st;
@@ -846,13 +1025,25 @@ xrt_status solve_zones(Context& c, const Graph& g, float obstacle_mass, float th
   const uint32_t n0 = off[1], n1 = off[2] - off[1], n2 = off[3] - off[2], n3 = off[4] - off[3];
   by_group[0] += n2;
   by_group[1] += n3;
-  if (n0) k_zone_solve<1, 1><<<n0, kZT, 0, s>>>(a, z.zid.p);
-  if (n1) k_zone_solve<kZoneCluster, 1><<<n1 * kZoneCluster, kZT, 0, s>>>(a, z.zid.p + off[1]);
+  // a launch whose zones all have at most one element per thread keeps them in registers
+  const uint32_t widest[4] = {kZT, kZoneCluster * kZT, kZoneClusterWide * kZT,
+                              kZoneClusterWide * kWideGroups * kZT};
+  bool one[4] = {true, true, true, true};
+  for (int g = 0; g < 4; ++g)
+    for (int32_t q : group[g])
+      one[g] &= (uint32_t)std::max(zone[q].y - zone[q].x, zone[q].w - zone[q].z) <= widest[g];
+  const int32_t* ids = z.zid.p;
+  if (n0) (one[0] ? k_zone_solve_one<1, 1> : k_zone_solve<1, 1>)<<<n0, kZT, 0, s>>>(a, ids);
+  if (n1)
+    (one[1] ? k_zone_solve_one<kZoneCluster, 1> : k_zone_solve<kZoneCluster, 1>)
+        <<<n1 * kZoneCluster, kZT, 0, s>>>(a, ids + off[1]);
   if (n2)
-    k_zone_solve<kZoneClusterWide, 1><<<n2 * kZoneClusterWide, kZT, 0, s>>>(a, z.zid.p + off[2]);
+    (one[2] ? k_zone_solve_one<kZoneClusterWide, 1> : k_zone_solve<kZoneClusterWide, 1>)
+        <<<n2 * kZoneClusterWide, kZT, 0, s>>>(a, ids + off[2]);
   if (n3)
-    k_zone_solve<kZoneClusterWide, kWideGroups><<<n3 * kZoneClusterWide, kWideGroups * kZT, 0, s>>>(
-        a, z.zid.p + off[3]);
+    (one[3] ? k_zone_solve_one<kZoneClusterWide, kWideGroups>
+            : k_zone_solve<kZoneClusterWide, kWideGroups>)
+        <<<n3 * kZoneClusterWide, kWideGroups * kZT, 0, s>>>(a, ids + off[3]);
   k_zone_finalize<<<nz, kZT, 0, s>>>(z.zone.p, z.conv.p, nz, z.znode.p, z.X.p, z.Xt.p, c.x.p,
                                      c.ox.p, c.nv);
   XRT_CUDA(&c, cudaGetLastError());
