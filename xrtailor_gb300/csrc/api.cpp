@@ -971,6 +971,7 @@ xrt_status xrt_start(xrt_ctx* h) {
       r.spacing = I.diameter * c.params.hash_cell_size;  // SpatialHashGPU: diameter x cell size
       r.spacing2 = r.spacing * r.spacing;
       r.d2 = I.diameter * I.diameter;
+      r.reach2 = xrt::reach_squared(I.diameter);
       r.table_base = tb;
       r.table_size = 2 * I.num_vertices;                  // table of 2V (SpatialHashGPU.cu:166)
       tb += r.table_size;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -165,7 +166,16 @@ struct InstanceRec {
   float spacing, spacing2, d2, diameter;  // hash cell size, its square, diameter^2, diameter
   uint32_t table_base, table_size;        // hash keys of the instance: [base, base + size)
   uint32_t vertex_base, num_vertices;     // cloth vertices
+  float reach2;  // the smallest float whose square root reaches the diameter
 };
+// Square roots round correctly and so do not decrease: sqrt(s) >= diameter exactly when s >= this.
+inline float reach_squared(float diameter) {
+  if (!(diameter > 0.0f)) return diameter == diameter ? 0.0f : diameter;
+  float s = diameter * diameter;
+  while (s > 0.0f && std::sqrt(s) >= diameter) s = std::nextafter(s, 0.0f);
+  while (std::sqrt(s) < diameter) s = std::nextafter(s, HUGE_VALF);
+  return s;
+}
 struct InstView {
   uint32_t count;
   const InstanceRec* rec;      // count records (unused when count == 1)
