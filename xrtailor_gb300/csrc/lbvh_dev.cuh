@@ -588,47 +588,4 @@ __device__ __forceinline__ uint32_t lbvh_traverse(const LbvhView& b, Overlap ov,
   return st.found;
 }
 
-// Persistent query loop with dynamic work fetch: every lane works on one query at a time and
-// takes a new one from `counter` when its query is done, so a warp's lanes stay busy while the
-// traversal lengths of neighbouring queries differ by orders of magnitude.  Lanes refill together
-// (one atomic per warp) once at least `kRefill` of them are idle.  A query is still processed by
-// exactly one lane, in the same order, so its result is that of a plain per-thread traversal.
-//   start(q)  -> bool:  set up query q, false = nothing to traverse (finish(q) still runs)
-//   step()    -> bool:  one traversal step of the lane's query, false = done
-//   finish(q):          write the result of query q
-template <class Start, class Step, class Finish>
-__device__ __forceinline__ void work_queue(uint32_t* counter, uint32_t nq, Start start, Step step,
-                                           Finish finish) {
-  constexpr unsigned kAll = 0xFFFFFFFFu;
-  constexpr int kRefill = 8;
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t q = kNone;
-  bool drained = false;  // the counter has passed nq
-  for (;;) {
-    const unsigned idle = __ballot_sync(kAll, q == kNone);
-    if (!drained && (idle == kAll || __popc(idle) >= kRefill)) {
-      const int leader = __ffs(idle) - 1;
-      uint32_t base = 0;
-      if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(idle));
-      base = __shfl_sync(kAll, base, leader);
-      if (base + (uint32_t)__popc(idle) >= nq) drained = true;
-      if (q == kNone) {
-        const uint32_t cand = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-        if (cand < nq) {
-          q = cand;
-          if (!start(q)) {
-            finish(q);
-            q = kNone;
-          }
-        }
-      }
-    }
-    if (__all_sync(kAll, q == kNone) && drained) break;
-    if (q != kNone && !step()) {
-      finish(q);
-      q = kNone;
-    }
-  }
-}
-
 }  // namespace xrt
