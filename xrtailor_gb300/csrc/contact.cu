@@ -88,35 +88,41 @@ __global__ void k_obstacle_commit(const float4* __restrict__ x, float4* __restri
 }
 
 // ---- contact generation: one query per cloth vertex (VF) or edge (EE) ------------------------------
-// Persistent warps whose lanes each walk the tree of their query's instance; lanes that are done
-// take new queries from a counter together, once kRefill of them are idle (walks near the obstacle
-// are hundreds of nodes long, the others end at the root).  A leaf's test is five to ten times a
-// box test and meets few lanes at a time, so the lanes only walk: the leaves go to a queue in
-// shared memory, and their tests run 32 at a time on full warps.  A query's result is the smallest
-// distance, and of equal ones that of the first leaf, kept as the minimum of (distance, place in
-// the walk) in one 64-bit word: the distances are not negative, so their bits compare as they do,
-// and a walk meets the leaves in the order of their tree positions.  The winner's data are computed
-// again at the end.  So each query tests the same nodes and leaves as in a walk by itself, with the
-// same cap, and the results are the same.  Contacts record global triangle ids.
-// Against walks that ran each leaf's test in place (7.7 of 32 lanes busy): 24 garments on bodies of
-// 13,776 triangles EE 740 -> 430 us, VF 340 -> 300 us; a 256 x 256 cloth EE 155 -> 75, VF 105 -> 72.
-// A warp walking the union of its lanes' nodes instead: 1,000 and 410 us, 95 and 78 us.
-constexpr int kGenWarps = kBlock / 32;
-constexpr int kRefill = 8;
+// A warp takes a packet of queries from a counter and works through (query, node) pairs: up to 32
+// pairs are taken off a stack in shared memory at a time, one a lane; a pair whose boxes overlap
+// puts the node's left child on the stack, and a left child its sibling.  So a query's walk is
+// spread over the lanes: walks near the obstacle are hundreds of nodes long and the others end at
+// the root, and a lane per query left a warp waiting for its longest.  The tests of the leaves, five
+// to ten box tests each, go to queues in shared memory and run 32 at a time as well.  A query's
+// result is the smallest distance, and of equal ones that of the first leaf of the walk, kept as the
+// minimum of (distance, tree position of the leaf) in one 64-bit word: the distances are not
+// negative, so their bits compare as they do, and a walk meets the leaves in the order of their
+// positions.  The winner's data are computed again at the end.  Only the cap of 256 leaves depends
+// on the order: queries that meet more are walked again, one a lane, in order, up to the cap.
+// Contacts record global triangle ids.
+// 24 garments on bodies of 13,776 triangles: EE 430 -> 251 us, VF 321 -> 107 against one walk per lane
+// with the same queues, and 740 / 340 us with the leaves' tests in the walk; a 256 x 256 cloth: EE 75
+// -> 43, VF 72 -> 30; an 11,495-vertex garment: EE 100 -> 33, VF 96 -> 30.  Bound by issue: about 190
+// instructions a round, most of them the segment's tests against the six faces.
+constexpr int kGenBlock = 128, kGenWarps = kGenBlock / 32;
+// Pairs on a warp's stack.  A full round leaves kReserve free; without room for one, pairs are taken
+// singly, which deepens the stack by at most one per level of the tree (64-bit keys: 65 levels).
+constexpr uint32_t kStack = 512, kReserve = 128;
 
-// A warp's queue of tests: x = element (global), y = place in the walk, z = lane that asks.
+// A warp's queue of tests: x = element (global), y = place in the walk, z = query that asks.
 template <int N>
 struct TestQueue {
   uint4 entry[N];
 };
-// Adds one test per lane with `on`; work(entry) runs 32 of them once there are as many.
+// Adds one test per lane with `on`; work(entry, true) runs 32 of them once there are as many.
 template <class Work>
 __device__ __forceinline__ void queue_push(TestQueue<64>& w, uint32_t& count, bool on,
-                                           uint32_t element, uint32_t place, Work work) {
+                                           uint32_t element, uint32_t place, uint32_t slot,
+                                           Work work) {
   const uint32_t lane = threadIdx.x & 31u;
   const unsigned m = __ballot_sync(0xFFFFFFFFu, on);
   if (m == 0) return;
-  if (on) w.entry[count + __popc(m & ((1u << lane) - 1u))] = make_uint4(element, place, lane, 0);
+  if (on) w.entry[count + __popc(m & ((1u << lane) - 1u))] = make_uint4(element, place, slot, 0);
   count += __popc(m);
   __syncwarp();
   if (count >= 32) {
@@ -129,13 +135,13 @@ __device__ __forceinline__ void queue_push(TestQueue<64>& w, uint32_t& count, bo
 // Runs what is left; work(entry, the lane has one).
 template <int N, class Work>
 __device__ __forceinline__ void queue_flush(TestQueue<N>& w, uint32_t& count, Work work) {
-  if (count == 0) return;
   const uint32_t lane = threadIdx.x & 31u;
   const bool on = lane < count;
   const uint4 e = on ? w.entry[lane] : make_uint4(0, 0, 0, 0);
+  __syncwarp();
+  if (count != 0) work(e, on);
   count = 0;
   __syncwarp();
-  work(e, on);
 }
 // The key of a result: smaller distances first, then the earlier place.  A distance counts only
 // below kScalarMax (no NaN, no infinity), so a key of no_result() stays where none does.
@@ -147,70 +153,97 @@ __device__ __forceinline__ void keep_nearest(unsigned long long& key, float dist
     atomicMin(&key, (unsigned long long)__float_as_uint(dist) << 32 | place);
 }
 
-// The loop of a warp: start(query) sets a lane's query up, step() visits one node on all lanes and
-// returns whether the lane's walk goes on, flush() runs the tests still queued, finish(query)
-// writes the result.
-template <class Start, class Step, class Flush, class Finish>
-__device__ __forceinline__ void query_loop(uint32_t* counter, uint32_t nq, Start start, Step step,
-                                           Flush flush, Finish finish) {
+struct PairStack {
+  uint2 e[kStack];      // node of the query's tree; query | left child << 5 | mask << 6
+  int4 tree[32];        // of each query: first node, primitives, first primitive
+};
+// Takes packets of `packet` queries until none of `nq` is left.  start(i) sets the lane's query up
+// and returns its mask of tests (0: none) and its tree's record; within(slot, mask) leaves the tests
+// of query `slot` that have not passed the cap, test(l, h, slot, mask) returns the
+// tests of query `slot` that overlap the box, leaf(hit, slot, element, place) takes the leaves of
+// all lanes (hit 0: none), finish(i, record) writes the lane's result.
+template <class Start, class Within, class Test, class Leaf, class Finish>
+__device__ __forceinline__ void pair_loop(PairStack& w, const LbvhForest& F, uint32_t* counter,
+                                          uint32_t nq, uint32_t packet, uint32_t* err, Start start,
+                                          Within within, Test test, Leaf leaf, Finish finish) {
   constexpr unsigned kAll = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t q = kNone;
-  bool walks = false, drained = false;  // drained: the counter has passed nq
+  const unsigned below = (1u << lane) - 1u;
   for (;;) {
-    const unsigned idle = __ballot_sync(kAll, !walks);
-    if (idle == kAll || (!drained && __popc(idle) >= kRefill)) {
-      flush();
-      __syncwarp();
-      if (!walks && q != kNone) {
-        finish(q);
-        q = kNone;
+    uint32_t first = 0;
+    if (lane == 0) first = atomicAdd(counter, packet);
+    first = __shfl_sync(kAll, first, 0);
+    if (first >= nq) return;
+    const uint32_t i = first + lane;
+    const bool valid = lane < packet && i < nq;
+    int4 rec = make_int4(0, 0, 0, 0);
+    const uint32_t mask = valid ? start(i, rec) : 0u;
+    w.tree[lane] = rec;
+    const bool has = mask != 0 && rec.y != 0;
+    const unsigned m = __ballot_sync(kAll, has);
+    if (has) w.e[__popc(m & below)] = make_uint2(0u, lane | mask << 6);
+    uint32_t count = __popc(m);
+    __syncwarp();
+    for (uint32_t guard = 0; count != 0; ++guard) {
+      uint32_t n = count < 32u ? count : 32u;
+      const uint32_t room = kStack - kReserve > count ? kStack - kReserve - count : 1u;
+      if (room < n) n = room;
+      if (guard / 32u > 2 * F.all.n + 2 || count > kStack - 2) {
+        raise_error(err, kErrTraversal);
+        break;
       }
-      if (drained) return;
-      uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(counter, (uint32_t)__popc(idle));
-      base = __shfl_sync(kAll, base, 0);
-      drained = base + (uint32_t)__popc(idle) >= nq;
-      const uint32_t cand = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-      if (!walks && cand < nq) {
-        q = cand;
-        walks = start(q);
-      }
+      count -= n;
+      const bool on = lane < n;
+      const uint2 e = on ? w.e[count + lane] : make_uint2(0, 0);
       __syncwarp();
+      const uint32_t slot = e.y & 31u, tests = on ? within(slot, e.y >> 6) : 0u;
+      uint32_t hit = 0, down = 0, esc = 0;
+      bool inner = false;
+      int4 t = make_int4(0, 0, 0, 0);
+      if (tests) {
+        t = w.tree[slot];
+        const float4 l = F.all.lo[t.z + (int)e.x], h = F.all.hi[t.z + (int)e.x];
+        down = (uint32_t)__float_as_int(l.w);
+        esc = (uint32_t)__float_as_int(h.w);
+        inner = (int)e.x < t.y - 1;
+        hit = test(l, h, slot, tests);
+      }
+      const bool deeper = inner && hit != 0, sibling = tests && (e.y & 32u);
+      const unsigned ms = __ballot_sync(kAll, sibling), md = __ballot_sync(kAll, deeper);
+      if (sibling) w.e[count + __popc(ms & below)] = make_uint2(esc, slot | tests << 6);
+      count += __popc(ms);
+      if (deeper) w.e[count + __popc(md & below)] = make_uint2(down, slot | 32u | hit << 6);
+      count += __popc(md);
+      __syncwarp();
+      leaf(inner ? 0u : hit, slot, (uint32_t)t.x + down, e.x - (uint32_t)(t.y - 1));
     }
-    walks = step(walks);
+    finish(valid, i, rec);
+    __syncwarp();
   }
 }
 
 // VF-DCD (nearest obstacle point of the predicted vertex) and VF-CCD (first obstacle hit of the
-// segment x0 -> x) of one vertex, in one walk of its instance's tree.  Each query keeps the state
-// of its own stackless traversal: where its box test fails at an internal node that the other
-// query enters, it stays off until the walk reaches that node's escape index (the first node
-// after the subtree), and it stops after its own 256th leaf.  So each query tests the same nodes
-// in the same order as alone, visits the same leaves in the same order and ends at the same cap:
-// both results are those of the two separate traversals (GenerateVF_DCD_Kernel,
+// segment x0 -> x) of one vertex, two tests of one query (GenerateVF_DCD_Kernel,
 // GenerateVFCCD_Kernel), with the nodes they share fetched once.
 struct VfShared {
+  PairStack stack;
   TestQueue<64> dq, cq;
   float4 x[32], x0[32], dir[32];  // dir.w = length
   unsigned long long dkey[32], ckey[32];
+  uint32_t found[32];  // leaves of the first test | of the second << 16
 };
-__global__ void __launch_bounds__(kBlock, 4) k_generate_vf(LbvhForest F, InstView I,
+__global__ void __launch_bounds__(kGenBlock) k_generate_vf(LbvhForest F, InstView I,
                                                         const float4* __restrict__ x,
                                                         const float4* __restrict__ x0,
                                                         uint32_t nv, int* __restrict__ vf_idx,
                                                         float4* __restrict__ vf_qs,
                                                         int* __restrict__ rt_idx,
                                                         float4* __restrict__ rt_qc, uint32_t* err,
-                                                        uint32_t* counter) {
-  constexpr int kOn = -1, kDone = -2;  // a query's state; >= 0: off until the walk reaches it
+                                                        uint32_t* counter, uint32_t packet) {
   __shared__ VfShared shared[kGenWarps];
   VfShared& w = shared[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31u;
-  LbvhView b{};
-  uint32_t base = 0, guard = 0, dfound = 0, cfound = 0, dcount = 0, ccount = 0;
-  int node = -1, dstate = kDone, cstate = kDone;
-  f3 px = mk3(0, 0, 0), p0 = px;
+  uint32_t dcount = 0, ccount = 0;
   auto nearest = [&](uint4 e, bool on) {
     if (!on) return;
     f3 qs;
@@ -224,81 +257,92 @@ __global__ void __launch_bounds__(kBlock, 4) k_generate_vf(LbvhForest F, InstVie
     keep_nearest(w.ckey[e.z],
                  ray_intersect(mk3(w.x0[e.z]), mk3(d), d.w, mk3(p[0]), mk3(p[1]), mk3(p[2])), e.y);
   };
-  query_loop(
-      counter, nv,
-      [&](uint32_t i) {
-        const uint32_t sg = inst_index(I, i);
-        b = forest_view(F, sg);
-        base = (uint32_t)forest_rec(F, sg).x;
-        px = mk3(x[i]);
-        p0 = mk3(x0[i]);
-        f3 dir = px - p0;
+  auto leaves = [&](uint32_t hit, uint32_t slot, uint32_t element, uint32_t place) {
+    queue_push(w.dq, dcount, hit & 1u, element, place, slot, nearest);
+    queue_push(w.cq, ccount, hit & 2u, element, place, slot, ray);
+  };
+  auto flush = [&]() {
+    queue_flush(w.dq, dcount, nearest);
+    queue_flush(w.cq, ccount, ray);
+  };
+  pair_loop(
+      w.stack, F, counter, nv, packet, err,
+      [&](uint32_t i, int4& rec) {
+        rec = forest_rec(F, inst_index(I, i));
+        const f3 p = mk3(x[i]), p0 = mk3(x0[i]);
+        f3 dir = p - p0;
         const float len = length(dir);
         const bool still = len < kEps;  // a still vertex casts no ray
         if (!still) dir = dir / len;
-        w.x[lane] = mk4(px, 0.0f);
+        w.x[lane] = mk4(p, 0.0f);
         w.x0[lane] = mk4(p0, 0.0f);
         w.dir[lane] = mk4(dir, len);
         w.dkey[lane] = w.ckey[lane] = no_result();
-        node = b.n == 0 ? -1 : 0;
-        guard = dfound = cfound = 0;
-        dstate = kOn;
-        cstate = still ? kDone : kOn;
-        return node != -1;
+        w.found[lane] = 0;
+        return still ? 1u : 3u;
       },
-      [&](bool on) {
-        bool od = false, oc = false, leaf = false;
-        uint32_t f = 0, place = 0;
-        if (on) {
-          if (dstate == node) dstate = kOn;  // the walk left the subtree the query skipped
-          if (cstate == node) cstate = kOn;
-          const bool don = dstate == kOn, con = cstate == kOn;
-          const float4 l = b.lo[node], h = b.hi[node];
-          od = don && overlap_point(l, h, px);
-          oc = con && overlap_segment(l, h, p0, px);
-          const int esc = __float_as_int(h.w), down = __float_as_int(l.w);
-          leaf = (uint32_t)node >= b.n - 1;
-          if (leaf) {
-            f = base + (uint32_t)down;
-            place = (uint32_t)node - (b.n - 1);
-            if (od && ++dfound >= kMaxCandidates) dstate = kDone;
-            if (oc && ++cfound >= kMaxCandidates) cstate = kDone;
-            node = esc;
-          } else if (od || oc) {
-            // off for the subtree (an escape of -1: for the rest of the walk)
-            if (don && !od) dstate = esc >= 0 ? esc : kDone;
-            if (con && !oc) cstate = esc >= 0 ? esc : kDone;
-            node = down;
-          } else {
-            node = esc;
+      [&](uint32_t slot, uint32_t mask) {
+        const uint32_t found = w.found[slot];
+        if ((found & 0xFFFFu) > kMaxCandidates) mask &= ~1u;
+        if (found >> 16 > kMaxCandidates) mask &= ~2u;
+        return mask;
+      },
+      [&](float4 l, float4 h, uint32_t slot, uint32_t mask) {
+        const f3 p = mk3(w.x[slot]);
+        uint32_t hit = (mask & 1u) && overlap_point(l, h, p) ? 1u : 0u;
+        if ((mask & 2u) && overlap_segment(l, h, mk3(w.x0[slot]), p)) hit |= 2u;
+        return hit;
+      },
+      [&](uint32_t hit, uint32_t slot, uint32_t element, uint32_t place) {
+        if (hit) atomicAdd(&w.found[slot], (hit & 1u) | (hit & 2u) << 15);
+        leaves(hit, slot, element, place);
+      },
+      [&](bool valid, uint32_t i, int4 rec) {
+        flush();
+        const LbvhView b{(uint32_t)rec.y, F.all.pred + 3 * (size_t)rec.x, F.all.lo + rec.z,
+                         F.all.hi + rec.z};
+        const f3 p = mk3(w.x[lane]), p0 = mk3(w.x0[lane]);
+        // beyond the cap: again in order, one walk per test
+#pragma unroll 1
+        for (uint32_t k = 1; k <= 2; ++k) {
+          const uint32_t found = k == 1 ? w.found[lane] & 0xFFFFu : w.found[lane] >> 16;
+          const bool again = valid && found > kMaxCandidates;
+          if (!__any_sync(0xFFFFFFFFu, again)) continue;
+          TraverseState st = lbvh_begin(b);
+          if (!again) st.node = -1;
+          else (k == 1 ? w.dkey[lane] : w.ckey[lane]) = no_result();
+          __syncwarp();
+          bool walks = true;
+          while (__any_sync(0xFFFFFFFFu, walks)) {
+            uint32_t f = kNone, place = 0;
+            const uint32_t at = (uint32_t)st.node;
+            walks = lbvh_step(
+                b, st,
+                [&](float4 l, float4 h) {
+                  return k == 1 ? overlap_point(l, h, p) : overlap_segment(l, h, p0, p);
+                },
+                [&](uint32_t o) {
+                  f = (uint32_t)rec.x + o;
+                  place = at - (b.n - 1);
+                },
+                err);
+            __syncwarp();
+            leaves(f != kNone ? k : 0u, lane, f, place);
           }
-          if (dstate == kDone && cstate == kDone) node = -1;
-          if (++guard > 2 * b.n + 2 && node != -1) {
-            raise_error(err, kErrTraversal);
-            node = -1;
-          }
+          flush();
         }
-        __syncwarp();
-        queue_push(w.dq, dcount, leaf && od, f, place, nearest);
-        queue_push(w.cq, ccount, leaf && oc, f, place, ray);
-        return on && node != -1;
-      },
-      [&]() {
-        queue_flush(w.dq, dcount, nearest);
-        queue_flush(w.cq, ccount, ray);
-      },
-      [&](uint32_t i) {
+        if (!valid) return;
         const unsigned long long d = w.dkey[lane], c = w.ckey[lane];
         f3 dqs = mk3(0, 0, 0), cqc = dqs;
         int didx = -1, cidx = -1;
         if (d != no_result()) {
           const int f = __float_as_int(b.lo[b.n - 1 + (uint32_t)d].w);
-          nearest_point(px, mk3(b.pred[3 * f]), mk3(b.pred[3 * f + 1]), mk3(b.pred[3 * f + 2]), dqs);
-          didx = (int)base + f;
+          nearest_point(p, mk3(b.pred[3 * f]), mk3(b.pred[3 * f + 1]), mk3(b.pred[3 * f + 2]), dqs);
+          didx = rec.x + f;
         }
         if (c != no_result()) {
           cqc = p0 + __uint_as_float((uint32_t)(c >> 32)) * mk3(w.dir[lane]);
-          cidx = (int)base + __float_as_int(b.lo[b.n - 1 + (uint32_t)c].w);
+          cidx = rec.x + __float_as_int(b.lo[b.n - 1 + (uint32_t)c].w);
         }
         vf_idx[i] = didx;
         vf_qs[i] = mk4(dqs, 0.0f);
@@ -311,12 +355,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_generate_vf(LbvhForest F, InstVie
 // queued leaves are taken apart 32 at a time into the edges they own (none to three), and those
 // are tested 32 at a time; element and place of an edge are three times the leaf's, plus its own.
 struct EeShared {
+  PairStack stack;
   TestQueue<64> leaves;
   TestQueue<128> edges;
   float4 p[32], q[32];
   unsigned long long key[32];
+  uint32_t found[32];
 };
-__global__ void __launch_bounds__(kBlock, 4) k_generate_ee(LbvhForest F, InstView I,
+__global__ void __launch_bounds__(kGenBlock) k_generate_ee(LbvhForest F, InstView I,
                                                         const float4* __restrict__ x,
                                                         const uint2* __restrict__ edge, uint32_t ne,
                                                         const int4* __restrict__ otri,
@@ -324,14 +370,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_generate_ee(LbvhForest F, InstVie
                                                         float4* __restrict__ ee_b,
                                                         float4* __restrict__ ee_c,
                                                         uint8_t* __restrict__ vflag, uint32_t* err,
-                                                        uint32_t* counter) {
+                                                        uint32_t* counter, uint32_t packet) {
   __shared__ EeShared shared[kGenWarps];
   EeShared& w = shared[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31u;
-  LbvhView b{};
-  uint32_t base = 0, guard = 0, found = 0, nleaf = 0, nedge = 0;
-  int node = -1;
-  f3 pc = mk3(0, 0, 0), qc = pc;
+  uint32_t nleaf = 0, nedge = 0;
   auto closest = [&](uint4 e, bool on) {
     if (!on) return;
     const uint32_t a = e.y % 3u;
@@ -358,51 +401,57 @@ __global__ void __launch_bounds__(kBlock, 4) k_generate_ee(LbvhForest F, InstVie
     }
     __syncwarp();
   };
-  query_loop(
-      counter, ne,
-      [&](uint32_t e) {
+  auto flush = [&]() {
+    queue_flush(w.leaves, nleaf, take_apart);
+    queue_flush(w.edges, nedge, closest);
+  };
+  pair_loop(
+      w.stack, F, counter, ne, packet, err,
+      [&](uint32_t e, int4& rec) {
         const uint2 ed = edge[e];
-        const uint32_t sg = inst_index(I, ed.x);
-        b = forest_view(F, sg);
-        base = (uint32_t)forest_rec(F, sg).x;
-        pc = mk3(x[ed.x]);
-        qc = mk3(x[ed.y]);
-        w.p[lane] = mk4(pc, 0.0f);
-        w.q[lane] = mk4(qc, 0.0f);
+        rec = forest_rec(F, inst_index(I, ed.x));
+        w.p[lane] = x[ed.x];
+        w.q[lane] = x[ed.y];
         w.key[lane] = no_result();
-        node = b.n == 0 ? -1 : 0;
-        guard = found = 0;
-        return node != -1;
+        w.found[lane] = 0;
+        return 1u;
       },
-      [&](bool on) {
-        bool hit = false;
-        uint32_t f = 0, place = 0;
-        if (on) {
-          const float4 l = b.lo[node], h = b.hi[node];
-          const bool ov = overlap_segment(l, h, pc, qc);
-          const int esc = __float_as_int(h.w), down = __float_as_int(l.w);
-          const bool leaf = (uint32_t)node >= b.n - 1;
-          if (ov && leaf) {
-            hit = true;
-            f = base + (uint32_t)down;
-            place = (uint32_t)node - (b.n - 1);
+      [&](uint32_t slot, uint32_t mask) { return w.found[slot] > kMaxCandidates ? 0u : mask; },
+      [&](float4 l, float4 h, uint32_t slot, uint32_t mask) {
+        return overlap_segment(l, h, mk3(w.p[slot]), mk3(w.q[slot])) ? 1u : 0u;
+      },
+      [&](uint32_t hit, uint32_t slot, uint32_t element, uint32_t place) {
+        if (hit) atomicAdd(&w.found[slot], 1u);
+        queue_push(w.leaves, nleaf, hit != 0, element, place, slot, take_apart);
+      },
+      [&](bool valid, uint32_t e, int4 rec) {
+        flush();
+        const LbvhView b{(uint32_t)rec.y, F.all.pred + 3 * (size_t)rec.x, F.all.lo + rec.z,
+                         F.all.hi + rec.z};
+        const bool again = valid && w.found[lane] > kMaxCandidates;
+        if (__any_sync(0xFFFFFFFFu, again)) {  // beyond the cap: again, in order
+          const f3 pc = mk3(w.p[lane]), qc = mk3(w.q[lane]);
+          TraverseState st = lbvh_begin(b);
+          if (!again) st.node = -1;
+          else w.key[lane] = no_result();
+          __syncwarp();
+          bool walks = true;
+          while (__any_sync(0xFFFFFFFFu, walks)) {
+            uint32_t f = kNone, place = 0;
+            const uint32_t at = (uint32_t)st.node;
+            walks = lbvh_step(
+                b, st, [&](float4 l, float4 h) { return overlap_segment(l, h, pc, qc); },
+                [&](uint32_t o) {
+                  f = (uint32_t)rec.x + o;
+                  place = at - (b.n - 1);
+                },
+                err);
+            __syncwarp();
+            queue_push(w.leaves, nleaf, f != kNone, f, place, lane, take_apart);
           }
-          node = ov && !leaf ? down : esc;
-          if (hit && ++found >= kMaxCandidates) node = -1;
-          if (++guard > 2 * b.n + 2 && node != -1) {
-            raise_error(err, kErrTraversal);
-            node = -1;
-          }
+          flush();
         }
-        __syncwarp();
-        queue_push(w.leaves, nleaf, hit, f, place, take_apart);
-        return on && node != -1;
-      },
-      [&]() {
-        queue_flush(w.leaves, nleaf, take_apart);
-        queue_flush(w.edges, nedge, closest);
-      },
-      [&](uint32_t e) {
+        if (!valid) return;
         const unsigned long long key = w.key[lane];
         float min_dist = kScalarMax, s = 0, t = 0;
         f3 p2 = mk3(0, 0, 0), q2 = p2, fn = p2;
@@ -414,7 +463,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_generate_ee(LbvhForest F, InstVie
           q2 = a == 0 ? v1 : a == 1 ? v2 : v0;
           fn = face_normal(v0, v1, v2);
           f3 c1, c2;
-          closest_seg_seg(pc, qc, p2, q2, s, t, c1, c2);
+          closest_seg_seg(mk3(w.p[lane]), mk3(w.q[lane]), p2, q2, s, t, c1, c2);
           min_dist = __uint_as_float((uint32_t)(key >> 32));
         }
         ee_a[e] = make_float4(min_dist, p2.x, p2.y, p2.z);
@@ -439,21 +488,35 @@ void launch_obstacle_pass(Context& c, int step, int num_steps) {
   launch_refit_midstep(c.bvh, c.ox1.p, c.on1.p, c.otri.p, c.params.bvh_tolerance, c.stream, c.err.p);
 }
 
+// Persistent warps: at most as many blocks as stay resident (six per SM) take packets until the
+// counter passes the end.  A large packet fills its warp's rounds; a small one is done sooner and
+// spreads the queries.  The largest with two packets per resident warp: of 11,495 / 33,950 queries
+// (VF / EE) packets of 32, 8, 4 take 37, 32, 30 / 57, 39, 33 us, of 65,536 / 195,841 queries packets
+// of 32, 16, 8, 4 take 32, 30, 30, 31 / 49, 43, 41, 45, of 0.9 / 2.7 M queries 32, 16, 8 take
+// 107, 132, 176 / 251, 317, 432.
+struct GenGrid {
+  unsigned blocks, packet;
+};
+static GenGrid gen_grid(const Context& c, uint32_t nq) {
+  const unsigned blocks = (unsigned)c.num_sms * 6u;
+  unsigned packet = 32;
+  while (packet > 4 && nq / packet < 2 * blocks * kGenWarps) packet /= 2;
+  return {std::min((nq - 1) / (packet * kGenWarps) + 1, blocks), packet};
+}
+
 void launch_generate_contacts(Context& c) {
   if (!c.bvh.active) return;
   const LbvhForest F = c.bvh.forest();
   const InstView I = c.inst_view();
-  // persistent work queues: a few resident waves of blocks fetch queries until the counters
-  // pass the end
-  const unsigned cap = (unsigned)c.num_sms * 8u;
   cudaMemsetAsync(c.gen_counter.p, 0, sizeof(uint32_t) * 3, c.stream);
   cudaMemsetAsync(c.ee_vflag.p, 0, c.nv, c.stream);  // this pass's contacts set it
-  k_generate_vf<<<std::min(grid_for(c.nv), cap), kBlock, 0, c.stream>>>(
-      F, I, c.x.p, c.x0.p, c.nv, c.vf_idx.p, c.vf_qs.p, c.rt_idx.p, c.rt_qc.p, c.err.p,
-      c.gen_counter.p);
-  k_generate_ee<<<std::min(grid_for(c.ne), cap), kBlock, 0, c.stream>>>(
-      F, I, c.x.p, c.edge.p, c.ne, c.otri.p, c.ee_a.p, c.ee_b.p, c.ee_c.p, c.ee_vflag.p, c.err.p,
-      c.gen_counter.p + 2);
+  const GenGrid v = gen_grid(c, c.nv), e = gen_grid(c, c.ne);
+  k_generate_vf<<<v.blocks, kGenBlock, 0, c.stream>>>(F, I, c.x.p, c.x0.p, c.nv, c.vf_idx.p,
+                                                      c.vf_qs.p, c.rt_idx.p, c.rt_qc.p, c.err.p,
+                                                      c.gen_counter.p, v.packet);
+  k_generate_ee<<<e.blocks, kGenBlock, 0, c.stream>>>(F, I, c.x.p, c.edge.p, c.ne, c.otri.p,
+                                                      c.ee_a.p, c.ee_b.p, c.ee_c.p, c.ee_vflag.p,
+                                                      c.err.p, c.gen_counter.p + 2, e.packet);
 }
 
 void launch_obstacle_commit(Context& c) {
