@@ -25,65 +25,103 @@ __device__ __forceinline__ f3 lerp_pos(const float4* __restrict__ x0, const floa
   return (1.0f - alpha) * mk3(x0[i]) + alpha * mk3(x[i]);
 }
 
-__global__ void k_obstacle_pass(const float4* __restrict__ x0, const float4* __restrict__ x,
-                                float4* __restrict__ x1, float4* __restrict__ n1,
-                                const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
-                                const uint32_t* __restrict__ list, uint32_t nv, float alpha) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  const f3 xi = lerp_pos(x0, x, i, alpha);
-  f3 acc = mk3(0, 0, 0);
-  for (uint32_t k = ptr[i]; k < ptr[i + 1]; ++k) {
-    const uint32_t fc = list[k];
-    const int4 t = tri[fc >> 2];
-    const int id[3] = {t.x, t.y, t.z};
-    const int j = (int)(fc & 3u);
-    const f3 e0 = lerp_pos(x0, x, id[(j + 1) % 3], alpha) - xi;
-    const f3 e1 = lerp_pos(x0, x, id[(j + 2) % 3], alpha) - xi;
-    acc = acc + cross(e0, e1) / (dot(e0, e0) * dot(e1, e1));
+// The weighted sum of the face normals around each vertex of the warp, in list order.  The warp's
+// vertices own consecutive entries of the list: the lanes work out the terms of kFan entries at a
+// time, one entry a lane, whichever vertex owns it, and each vertex adds its own up from shared
+// memory.  A vertex has six faces as a rule, but a pole of a body of revolution its whole ring, and a
+// lane that takes its vertex's faces one after the other takes 27 us for a ring of 84.
+// 6,890 vertices with such poles: 29 -> 9.4 us, 165,360 of them 44 -> 22 us; without poles 4,096 vertices
+// take 9.8 us against 7.7 and 642 take 8.1 against 7.5 (the owner's position is read once more per
+// face).
+constexpr int kFanBlock = 64;
+constexpr uint32_t kFanRounds = 6, kFan = 32 * kFanRounds;
+struct FanShared {
+  float x[kFan], y[kFan], z[kFan];
+};
+template <class Pos>
+__device__ __forceinline__ f3 fan_sum(FanShared& w, const int4* __restrict__ tri,
+                                      const uint32_t* __restrict__ ptr,
+                                      const uint32_t* __restrict__ list, uint32_t i, uint32_t nv,
+                                      Pos pos) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t k = 0, end = 0;
+  if (i < nv) {
+    k = ptr[i];
+    end = ptr[i + 1];
   }
-  x1[i] = mk4(xi, 0.0f);
+  const uint32_t first = __shfl_sync(0xFFFFFFFFu, k, 0);
+  const uint32_t last = __reduce_max_sync(0xFFFFFFFFu, end);
+  f3 acc = mk3(0, 0, 0);
+  for (uint32_t base = first; base < last; base += kFan) {
+    const uint32_t n = min(last - base, kFan);
+    uint32_t fc[kFanRounds];
+    int4 t[kFanRounds];
+    f3 xi[kFanRounds], e0[kFanRounds], e1[kFanRounds];
+#pragma unroll
+    for (uint32_t r = 0; r < kFanRounds; ++r)
+      fc[r] = 32 * r + lane < n ? list[base + 32 * r + lane] : 0u;
+#pragma unroll
+    for (uint32_t r = 0; r < kFanRounds; ++r)
+      if (32 * r + lane < n) t[r] = tri[fc[r] >> 2];
+#pragma unroll
+    for (uint32_t r = 0; r < kFanRounds; ++r) {
+      if (32 * r + lane >= n) continue;
+      const uint32_t j = fc[r] & 3u;  // the owner's corner
+      xi[r] = pos(j == 0 ? t[r].x : j == 1 ? t[r].y : t[r].z);
+      e0[r] = pos(j == 0 ? t[r].y : j == 1 ? t[r].z : t[r].x);
+      e1[r] = pos(j == 0 ? t[r].z : j == 1 ? t[r].x : t[r].y);
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < kFanRounds; ++r) {
+      if (32 * r + lane >= n) continue;
+      const f3 a = e0[r] - xi[r], b = e1[r] - xi[r];
+      const f3 term = cross(a, b) / (dot(a, a) * dot(b, b));
+      w.x[32 * r + lane] = term.x;
+      w.y[32 * r + lane] = term.y;
+      w.z[32 * r + lane] = term.z;
+    }
+    __syncwarp();
+    for (; k < end && k < base + n; ++k)
+      acc = acc + mk3(w.x[k - base], w.y[k - base], w.z[k - base]);
+    __syncwarp();
+  }
+  return acc;
+}
+
+__global__ void __launch_bounds__(kFanBlock) k_obstacle_pass(
+    const float4* __restrict__ x0, const float4* __restrict__ x, float4* __restrict__ x1,
+    float4* __restrict__ n1, const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
+    const uint32_t* __restrict__ list, uint32_t nv, float alpha) {
+  __shared__ FanShared shared[kFanBlock / 32];
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const f3 acc = fan_sum(shared[threadIdx.x >> 5], tri, ptr, list, i, nv,
+                         [&](int j) { return lerp_pos(x0, x, j, alpha); });
+  if (i >= nv) return;
+  x1[i] = mk4(lerp_pos(x0, x, i, alpha), 0.0f);
   n1[i] = mk4(normalize(acc), 0.0f);
 }
 
-__global__ void k_vertex_normals(const float4* __restrict__ x, const int4* __restrict__ tri,
-                                 const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ list,
-                                 float4* __restrict__ out, uint32_t nv) {
+__global__ void __launch_bounds__(kFanBlock) k_vertex_normals(
+    const float4* __restrict__ x, const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
+    const uint32_t* __restrict__ list, float4* __restrict__ out, uint32_t nv) {
+  __shared__ FanShared shared[kFanBlock / 32];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  const f3 xi = mk3(x[i]);
-  f3 acc = mk3(0, 0, 0);
-  for (uint32_t k = ptr[i]; k < ptr[i + 1]; ++k) {
-    const uint32_t fc = list[k];
-    const int4 t = tri[fc >> 2];
-    const int id[3] = {t.x, t.y, t.z};
-    const int j = (int)(fc & 3u);
-    const f3 e0 = mk3(x[id[(j + 1) % 3]]) - xi;
-    const f3 e1 = mk3(x[id[(j + 2) % 3]]) - xi;
-    acc = acc + cross(e0, e1) / (dot(e0, e0) * dot(e1, e1));
-  }
-  out[i] = mk4(normalize(acc), 0.0f);
+  const f3 acc = fan_sum(shared[threadIdx.x >> 5], tri, ptr, list, i, nv,
+                         [&](int j) { return mk3(x[j]); });
+  if (i < nv) out[i] = mk4(normalize(acc), 0.0f);
 }
 
 // Frame end: x0 = x, then normals of the new x0 (computed from x, which is the same data).
-__global__ void k_obstacle_commit(const float4* __restrict__ x, float4* __restrict__ x0,
-                                  float4* __restrict__ nrm, const int4* __restrict__ tri,
-                                  const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ list,
-                                  uint32_t nv) {
+__global__ void __launch_bounds__(kFanBlock) k_obstacle_commit(
+    const float4* __restrict__ x, float4* __restrict__ x0, float4* __restrict__ nrm,
+    const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
+    const uint32_t* __restrict__ list, uint32_t nv) {
+  __shared__ FanShared shared[kFanBlock / 32];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const f3 acc = fan_sum(shared[threadIdx.x >> 5], tri, ptr, list, i, nv,
+                         [&](int j) { return mk3(x[j]); });
   if (i >= nv) return;
-  const f3 xi = mk3(x[i]);
-  f3 acc = mk3(0, 0, 0);
-  for (uint32_t k = ptr[i]; k < ptr[i + 1]; ++k) {
-    const uint32_t fc = list[k];
-    const int4 t = tri[fc >> 2];
-    const int id[3] = {t.x, t.y, t.z};
-    const int j = (int)(fc & 3u);
-    const f3 e0 = mk3(x[id[(j + 1) % 3]]) - xi;
-    const f3 e1 = mk3(x[id[(j + 2) % 3]]) - xi;
-    acc = acc + cross(e0, e1) / (dot(e0, e0) * dot(e1, e1));
-  }
-  x0[i] = mk4(xi, 0.0f);
+  x0[i] = mk4(mk3(x[i]), 0.0f);
   nrm[i] = mk4(normalize(acc), 0.0f);
 }
 
@@ -482,7 +520,7 @@ __global__ void __launch_bounds__(kGenBlock) k_generate_ee(LbvhForest F, InstVie
 void launch_obstacle_pass(Context& c, int step, int num_steps) {
   if (c.onv == 0) return;
   const float alpha = ((float)step + 1.0f) / (float)num_steps;
-  k_obstacle_pass<<<grid_for(c.onv), kBlock, 0, c.stream>>>(c.ox0.p, c.ox.p, c.ox1.p, c.on1.p,
+  k_obstacle_pass<<<grid_for(c.onv, kFanBlock), kFanBlock, 0, c.stream>>>(c.ox0.p, c.ox.p, c.ox1.p, c.on1.p,
                                                             c.otri.p, c.ovf_ptr.p, c.ovf_list.p,
                                                             c.onv, alpha);
   launch_refit_midstep(c.bvh, c.ox1.p, c.on1.p, c.otri.p, c.params.bvh_tolerance, c.stream, c.err.p);
@@ -521,14 +559,14 @@ void launch_generate_contacts(Context& c) {
 
 void launch_obstacle_commit(Context& c) {
   if (c.onv == 0) return;
-  k_obstacle_commit<<<grid_for(c.onv), kBlock, 0, c.stream>>>(c.ox.p, c.ox0.p, c.on.p, c.otri.p,
+  k_obstacle_commit<<<grid_for(c.onv, kFanBlock), kFanBlock, 0, c.stream>>>(c.ox.p, c.ox0.p, c.on.p, c.otri.p,
                                                               c.ovf_ptr.p, c.ovf_list.p, c.onv);
 }
 
 void launch_vertex_normals(const float4* x, const int4* tri, const uint32_t* ptr,
                            const uint32_t* list, float4* out, uint32_t nv, cudaStream_t s) {
   if (nv == 0) return;
-  k_vertex_normals<<<grid_for(nv), kBlock, 0, s>>>(x, tri, ptr, list, out, nv);
+  k_vertex_normals<<<grid_for(nv, kFanBlock), kFanBlock, 0, s>>>(x, tri, ptr, list, out, nv);
 }
 
 void launch_prims_obstacle(Context& c, float tol) {
