@@ -410,7 +410,7 @@ xrt_status xrt_destroy(xrt_ctx* h) {
     cudaEventDestroy(e.b);
   }
   DBuf<float4>* f4[] = {&c.x, &c.x_alt, &c.x0, &c.v, &c.n, &c.x_init, &c.bind_a, &c.vf_qs,
-                        &c.rt_qc, &c.ee_a, &c.ee_b, &c.ee_c, &c.ox0, &c.ox, &c.ox1, &c.on, &c.on1};
+                        &c.rt_qc, &c.vf_ns, &c.rt_nc, &c.ee_a, &c.ee_b, &c.ee_c, &c.ee_rec, &c.ox0, &c.ox, &c.ox1, &c.on, &c.on1};
   for (auto* b : f4) b->release();
   DBuf<uint32_t>* u[] = {&c.vf_ptr, &c.vf_list, &c.lra_ptr, &c.lra_src, &c.lra_l_src, &c.lra_l_tgt,
                          &c.bind_ptr, &c.ve_ptr, &c.ve_list, &c.hash_key, &c.hash_val,
@@ -421,7 +421,7 @@ xrt_status xrt_destroy(xrt_ctx* h) {
   c.s_lambda.release(); c.lra_rest.release(); c.lra_l_rest.release(); c.b_tc.release();
   c.stage3.release();
   c.ee_vflag.release();
-  c.edge.release(); c.vf_idx.release(); c.rt_idx.release();
+  c.edge.release(); c.ve_pair.release(); c.vf_idx.release(); c.rt_idx.release();
   c.hash_sorter.keys_tmp.release(); c.hash_sorter.vals_tmp.release(); c.hash_sorter.hist.release();
   c.hash_sorter.sums.release();
   c.bvh.release();
@@ -1064,6 +1064,10 @@ xrt_status xrt_start(xrt_ctx* h) {
   xrt::setup::build_ve(c.h_edges, c.nv, ptr, list);
   XRT_CUDA(&c, upload(c.ve_ptr, ptr, c.stream));
   XRT_CUDA(&c, upload(c.ve_list, list, c.stream));
+  std::vector<uint2> pair(list.size());
+  for (size_t k = 0; k < list.size(); ++k)
+    pair[k] = make_uint2(list[k], c.h_edges[(size_t)list[k] ^ 1u]);
+  XRT_CUDA(&c, upload(c.ve_pair, pair, c.stream));
   xrt::launch_vertex_normals(c.x0.p, c.tri.p, c.vf_ptr.p, c.vf_list.p, c.n.p, c.nv, c.stream);
   // LRA: by target when every slot vertex is pinned, else slot-major blocks
   {
@@ -1102,9 +1106,12 @@ xrt_status xrt_start(xrt_ctx* h) {
   XRT_CUDA(&c, c.rt_idx.reserve(c.nv));
   XRT_CUDA(&c, c.vf_qs.reserve(c.nv));
   XRT_CUDA(&c, c.rt_qc.reserve(c.nv));
+  XRT_CUDA(&c, c.vf_ns.reserve(c.nv));
+  XRT_CUDA(&c, c.rt_nc.reserve(c.nv));
   XRT_CUDA(&c, c.ee_a.reserve(std::max(c.ne, 1u)));
   XRT_CUDA(&c, c.ee_b.reserve(std::max(c.ne, 1u)));
   XRT_CUDA(&c, c.ee_c.reserve(std::max(c.ne, 1u)));
+  XRT_CUDA(&c, c.ee_rec.reserve(2 * (size_t)std::max(c.ne, 1u)));
   XRT_CUDA(&c, c.ee_vflag.reserve(std::max(c.nv, 1u)));
   XRT_CUDA(&c, cudaMemsetAsync(c.ee_vflag.p, 0, std::max(c.nv, 1u), c.stream));
   XRT_CUDA(&c, cudaMemsetAsync(c.vf_idx.p, 0xFF, sizeof(int) * c.nv, c.stream));

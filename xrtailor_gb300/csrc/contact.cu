@@ -275,8 +275,10 @@ __global__ void __launch_bounds__(kGenBlock) k_generate_vf(LbvhForest F, InstVie
                                                         const float4* __restrict__ x0,
                                                         uint32_t nv, int* __restrict__ vf_idx,
                                                         float4* __restrict__ vf_qs,
+                                                        float4* __restrict__ vf_ns,
                                                         int* __restrict__ rt_idx,
-                                                        float4* __restrict__ rt_qc, uint32_t* err,
+                                                        float4* __restrict__ rt_qc,
+                                                        float4* __restrict__ rt_nc, uint32_t* err,
                                                         uint32_t* counter, uint32_t packet) {
   __shared__ VfShared shared[kGenWarps];
   VfShared& w = shared[threadIdx.x >> 5];
@@ -375,12 +377,17 @@ __global__ void __launch_bounds__(kGenBlock) k_generate_vf(LbvhForest F, InstVie
         int didx = -1, cidx = -1;
         if (d != no_result()) {
           const int f = __float_as_int(b.lo[b.n - 1 + (uint32_t)d].w);
-          nearest_point(p, mk3(b.pred[3 * f]), mk3(b.pred[3 * f + 1]), mk3(b.pred[3 * f + 2]), dqs);
+          const f3 v0 = mk3(b.pred[3 * f]), v1 = mk3(b.pred[3 * f + 1]), v2 = mk3(b.pred[3 * f + 2]);
+          nearest_point(p, v0, v1, v2, dqs);
           didx = rec.x + f;
+          vf_ns[i] = mk4(face_normal(v0, v1, v2), 0.0f);
         }
         if (c != no_result()) {
           cqc = p0 + __uint_as_float((uint32_t)(c >> 32)) * mk3(w.dir[lane]);
-          cidx = rec.x + __float_as_int(b.lo[b.n - 1 + (uint32_t)c].w);
+          const int f = __float_as_int(b.lo[b.n - 1 + (uint32_t)c].w);
+          cidx = rec.x + f;
+          rt_nc[i] = mk4(face_normal(mk3(b.pred[3 * f]), mk3(b.pred[3 * f + 1]),
+                                     mk3(b.pred[3 * f + 2])), 0.0f);
         }
         vf_idx[i] = didx;
         vf_qs[i] = mk4(dqs, 0.0f);
@@ -407,6 +414,7 @@ __global__ void __launch_bounds__(kGenBlock) k_generate_ee(LbvhForest F, InstVie
                                                         float4* __restrict__ ee_a,
                                                         float4* __restrict__ ee_b,
                                                         float4* __restrict__ ee_c,
+                                                        float4* __restrict__ ee_rec,
                                                         uint8_t* __restrict__ vflag, uint32_t* err,
                                                         uint32_t* counter, uint32_t packet) {
   __shared__ EeShared shared[kGenWarps];
@@ -507,6 +515,9 @@ __global__ void __launch_bounds__(kGenBlock) k_generate_ee(LbvhForest F, InstVie
         ee_a[e] = make_float4(min_dist, p2.x, p2.y, p2.z);
         ee_b[e] = make_float4(q2.x, q2.y, q2.z, s);
         ee_c[e] = make_float4(fn.x, fn.y, fn.z, t);
+        const f3 c2 = (1 - t) * p2 + t * q2;
+        ee_rec[2 * (size_t)e] = make_float4(c2.x, c2.y, c2.z, s);
+        ee_rec[2 * (size_t)e + 1] = make_float4(fn.x, fn.y, fn.z, min_dist);
         if (min_dist <= 1e6f) {  // a contact (the EE solve's test): flag both endpoints
           const uint2 ed = edge[e];
           vflag[ed.x] = 1;
@@ -550,10 +561,12 @@ void launch_generate_contacts(Context& c) {
   cudaMemsetAsync(c.ee_vflag.p, 0, c.nv, c.stream);  // this pass's contacts set it
   const GenGrid v = gen_grid(c, c.nv), e = gen_grid(c, c.ne);
   k_generate_vf<<<v.blocks, kGenBlock, 0, c.stream>>>(F, I, c.x.p, c.x0.p, c.nv, c.vf_idx.p,
-                                                      c.vf_qs.p, c.rt_idx.p, c.rt_qc.p, c.err.p,
+                                                      c.vf_qs.p, c.vf_ns.p, c.rt_idx.p, c.rt_qc.p,
+                                                      c.rt_nc.p, c.err.p,
                                                       c.gen_counter.p, v.packet);
   k_generate_ee<<<e.blocks, kGenBlock, 0, c.stream>>>(F, I, c.x.p, c.edge.p, c.ne, c.otri.p,
-                                                      c.ee_a.p, c.ee_b.p, c.ee_c.p, c.ee_vflag.p,
+                                                      c.ee_a.p, c.ee_b.p, c.ee_c.p, c.ee_rec.p,
+                                                      c.ee_vflag.p,
                                                       c.err.p, c.gen_counter.p + 2, e.packet);
 }
 

@@ -500,10 +500,13 @@ struct Context {
   DBuf<int4> bind_b;                 // iu, iv, iw, stiffness bits
   DBuf<uint2> edge;                  // original edge order (EE contacts)
   DBuf<uint32_t> ve_ptr, ve_list;    // vertex -> (edge << 1 | side), ascending edges
+  DBuf<uint2> ve_pair;               // {entry of ve_list, the edge's other vertex}
   // contacts
   DBuf<int> vf_idx, rt_idx;
   DBuf<float4> vf_qs, rt_qc;
+  DBuf<float4> vf_ns, rt_nc;         // normals of the triangles vf_idx / rt_idx, where there is one
   DBuf<float4> ee_a, ee_b, ee_c;     // {dist, p2}, {q2, s}, {fn, t}
+  DBuf<float4> ee_rec;               // per edge {obstacle point, s}, {fn, dist}: what the solve reads
   // particle hash
   DBuf<uint32_t> hash_key, hash_val, cell_start, cell_end, neighbors;
   DBuf<float> stage3;  // packed xyz staging of the C ABI's host copies

@@ -383,10 +383,10 @@ struct TailArgs {
   const float* lra_rest;
   float lra_stretch;
   const int *rt_idx, *vf_idx;
-  const float4 *rt_qc, *vf_qs, *pred;
-  const uint32_t *ve_ptr, *ve_list;
-  const uint2* edge;
-  const float4 *ee_a, *ee_b, *ee_c;
+  const float4 *rt_qc, *rt_nc, *vf_qs, *vf_ns;
+  const uint32_t* ve_ptr;
+  const uint2* ve_pair;
+  const float4* ee_rec;
   const uint8_t* ee_vflag;  // per vertex: an incident edge holds a contact
   float relaxation;
   const uint32_t* bind_ptr;
@@ -397,70 +397,88 @@ struct TailArgs {
   float* tape_cnt;  // TAPE, k_ee: each vertex's EE contact count
 };
 
-// Position of vertex j after the LRA and VF phases.
-template <bool LRA, bool CONTACTS>
-__device__ __forceinline__ f3 tail_stage(const TailArgs& a, uint32_t j, const float4 p) {
-  f3 q = mk3(p);
-  if (LRA) {
-    const uint32_t b = __ldg(&a.lra_ptr[j]), e = __ldg(&a.lra_ptr[j + 1]);
-    if (b != e) {
-      f3 xt = q;
-      for (uint32_t k = b; k < e; ++k)
-        xt = lra_project(xt, mk3(a.x_in[__ldg(&a.lra_src[k])]), p.w, __ldg(&a.lra_rest[k]),
-                         a.lra_stretch);
-      if (xt.x != p.x || xt.y != p.y || xt.z != p.z) q = xt;  // the phase writes only changes
-    }
-  }
-  if (CONTACTS) {
-    const int rc = a.rt_idx[j], vc = a.vf_idx[j];
-    if (rc != -1) {
-      const f3 nc = prim_normal(a.pred, rc);
-      const float lambda = dot(nc, q - mk3(a.rt_qc[j]));
-      if (lambda < 0) q = q + (-lambda * nc);
-    }
-    if (vc != -1) {
-      const f3 ns = prim_normal(a.pred, vc);
-      const float lambda = dot(ns, q - mk3(a.vf_qs[j])) - 1e-3f;
-      if (lambda < 0) q = q + (-lambda * ns);
-    }
-  }
-  return q;
-}
-
-// LRA + VF: x_out = tail_stage(x_in), per vertex.
-template <bool LRA, bool CONTACTS, bool TAPE>
+// LRA + VF, per vertex.  AHEAD: the slots' lists (setup-time) are read ahead of the wait, and their
+// positions in one round with the vertex's own and the contacts' triangles; a second round brings
+// the contacts, with the normals their generation stored (computed here from the triangle's
+// corners before: 6.0 -> 5.2 us at 65,536 vertices, two slots).  At 917 k vertices AHEAD is 18.2 us
+// against 17.0 without.
+template <bool LRA, bool CONTACTS, bool TAPE, bool AHEAD>
 __global__ void k_stage(const TailArgs a) {
   pdl_release();
-  pdl_wait();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int kSlots = 2;
+  uint32_t b = 0, e = 0, src[kSlots];
+  float rest[kSlots];
+  f3 anchor[kSlots];
+  if (LRA && i < a.nv) {
+    b = __ldg(&a.lra_ptr[i]);
+    e = __ldg(&a.lra_ptr[i + 1]);
+    if (AHEAD) {
+#pragma unroll
+      for (int r = 0; r < kSlots; ++r) {
+        src[r] = b + r < e ? __ldg(&a.lra_src[b + r]) : 0u;
+        rest[r] = b + r < e ? __ldg(&a.lra_rest[b + r]) : 0.0f;
+      }
+    }
+  }
+  pdl_wait();
   if (i >= a.nv) return;
   const float4 p = a.x_in[i];
+  const int rc = CONTACTS ? a.rt_idx[i] : -1, vc = CONTACTS ? a.vf_idx[i] : -1;
+  if (LRA && AHEAD) {
+#pragma unroll
+    for (int r = 0; r < kSlots; ++r)
+      if (b + r < e) anchor[r] = mk3(a.x_in[src[r]]);
+  }
+  float4 qc, nc, qs, ns;
+  if (rc != -1) {
+    qc = a.rt_qc[i];
+    nc = a.rt_nc[i];
+  }
+  if (vc != -1) {
+    qs = a.vf_qs[i];
+    ns = a.vf_ns[i];
+  }
   if (TAPE) a.tape[i] = p;
-  a.x_out[i] = mk4(tail_stage<LRA, CONTACTS>(a, i, p), p.w);
+  f3 q = mk3(p);
+  if (LRA && b != e) {
+    f3 xt = q;
+    if (AHEAD) {
+#pragma unroll
+      for (int r = 0; r < kSlots; ++r)
+        if (b + r < e) xt = lra_project(xt, anchor[r], p.w, rest[r], a.lra_stretch);
+    }
+    for (uint32_t k = b + (AHEAD ? kSlots : 0); k < e; ++k)
+      xt = lra_project(xt, mk3(a.x_in[__ldg(&a.lra_src[k])]), p.w, __ldg(&a.lra_rest[k]),
+                       a.lra_stretch);
+    if (xt.x != p.x || xt.y != p.y || xt.z != p.z) q = xt;  // the phase writes only changes
+  }
+  if (rc != -1) {
+    const float lambda = dot(mk3(nc), q - mk3(qc));
+    if (lambda < 0) q = q + (-lambda * mk3(nc));
+  }
+  if (vc != -1) {
+    const float lambda = dot(mk3(ns), q - mk3(qs)) - 1e-3f;
+    if (lambda < 0) q = q + (-lambda * mk3(ns));
+  }
+  a.x_out[i] = mk4(q, p.w);
 }
 
-// EE + ApplyDeltas + binding on the post-VF positions x_in.
+// EE + ApplyDeltas + binding on the post-VF positions x_in.  The flagged vertices read their edges
+// with the other ends, then the records and positions of kBatch edges together; the edges are then
+// processed in list order.  Per edge one record and one position, against three records, two ends
+// and three loads one behind the other before: 7.3 -> 6.5 us at 65,536 vertices in contact, 8.4 -> 7.2
+// at 538,368.  Reading every vertex's list ahead of the wait: no faster at 65,536, 28 us against 20 at
+// 917 k vertices.
 template <bool CONTACTS, bool BINDINGS, bool TAPE>
 __global__ void k_ee(const TailArgs a) {
   pdl_release();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t nv = a.nv;
-  // incident-edge list (setup-time) ahead of the wait
-  constexpr int kBatch = 8;
-  uint32_t kb = 0, ke = 0, code[kBatch];
-  if (CONTACTS && i < nv) {
-    kb = __ldg(&a.ve_ptr[i]);
-    ke = __ldg(&a.ve_ptr[i + 1]);
-#pragma unroll
-    for (int r = 0; r < kBatch; ++r) code[r] = kb + r < ke ? __ldg(&a.ve_list[kb + r]) : 0u;
-  }
   pdl_wait();
   if (i >= nv) return;
   const float4* __restrict__ x_in = a.x_in;
-  const float4* __restrict__ ee_a = a.ee_a;
-  const float4* __restrict__ ee_b = a.ee_b;
-  const float4* __restrict__ ee_c = a.ee_c;
-  const uint32_t* __restrict__ ve_list = a.ve_list;
+  const float4* __restrict__ rec = a.ee_rec;
   const float relaxation = a.relaxation;
   const float4 p = x_in[i];
   if (TAPE) a.tape[i] = p;
@@ -469,34 +487,39 @@ __global__ void k_ee(const TailArgs a) {
   // a vertex none of whose edges holds a contact skips the list (delta 0, count 0)
   if (CONTACTS && a.ee_vflag[i]) {
     f3 delta = mk3(0, 0, 0);
-    // The contact-flag loads of a batch of incident edges are issued together; the edges are
-    // then processed one by one in list order.
-    for (uint32_t base = kb; base < ke; base += kBatch) {
-      if (base != kb) {
+    constexpr int kBatch = 4;
+    const uint32_t end = __ldg(&a.ve_ptr[i + 1]);
+    for (uint32_t base = __ldg(&a.ve_ptr[i]); base < end; base += kBatch) {
+      uint2 pair[kBatch];
+      float4 r0[kBatch], r1[kBatch];
+      f3 xo[kBatch];
 #pragma unroll
-        for (int r = 0; r < kBatch; ++r) code[r] = base + r < ke ? ve_list[base + r] : 0u;
-      }
-      float flag[kBatch];
-#pragma unroll
-      for (int r = 0; r < kBatch; ++r) flag[r] = base + r < ke ? ee_a[code[r] >> 1].x : 2e6f;
+      for (int r = 0; r < kBatch; ++r)
+        pair[r] = base + r < end ? __ldg(&a.ve_pair[base + r]) : make_uint2(0, 0);
 #pragma unroll
       for (int r = 0; r < kBatch; ++r) {
-        if (flag[r] > 1e6f) continue;  // no contact on this edge (or past the list)
-        const uint32_t e = code[r] >> 1;
-        const float4 ca = ee_a[e];
-        const float4 cb = ee_b[e], cc = ee_c[e];
-        const uint2 ed = a.edge[e];
-        const f3 p1 = mk3(x_in[ed.x]), q1 = mk3(x_in[ed.y]);
-        const float s = cb.w, t = cc.w;
-        const f3 fn = mk3(cc);
+        const size_t e = pair[r].x >> 1;
+        r1[r].w = 2e6f;
+        if (base + r < end) {
+          r0[r] = rec[2 * e];
+          r1[r] = rec[2 * e + 1];
+          xo[r] = mk3(x_in[pair[r].y]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kBatch; ++r) {
+        if (r1[r].w > 1e6f) continue;  // no contact on this edge (or past the list)
+        const bool second = pair[r].x & 1u;  // the vertex is the edge's second end
+        const f3 p1 = second ? xo[r] : mk3(p), q1 = second ? mk3(p) : xo[r];
+        const float s = r0[r].w;
+        const f3 fn = mk3(r1[r]);
         const f3 c1 = (1 - s) * p1 + s * q1;
-        const f3 c2 = (1 - t) * mk3(ca.y, ca.z, ca.w) + t * mk3(cb);
-        const f3 d = c1 - c2;
+        const f3 d = c1 - mk3(r0[r]);
         const float len = length(d);
         if (len < kEps) continue;
         const float lambda = dot(d, fn) - 1e-3f;
         if (lambda > 0) continue;
-        const f3 corr = (code[r] & 1u) ? (-(s)*lambda * fn) : (-(1 - s) * lambda * fn);
+        const f3 corr = second ? (-(s)*lambda * fn) : (-(1 - s) * lambda * fn);
         delta = delta + corr;
         ++count;
       }
@@ -753,13 +776,11 @@ static TailArgs tail_args(Context& c, const FrameConst& k) {
   a.vf_idx = c.vf_idx.p;
   a.rt_qc = c.rt_qc.p;
   a.vf_qs = c.vf_qs.p;
-  a.pred = c.bvh.pred.p;
+  a.rt_nc = c.rt_nc.p;
+  a.vf_ns = c.vf_ns.p;
   a.ve_ptr = c.ve_ptr.p;
-  a.ve_list = c.ve_list.p;
-  a.edge = c.edge.p;
-  a.ee_a = c.ee_a.p;
-  a.ee_b = c.ee_b.p;
-  a.ee_c = c.ee_c.p;
+  a.ve_pair = c.ve_pair.p;
+  a.ee_rec = c.ee_rec.p;
   a.ee_vflag = c.ee_vflag.p;
   a.relaxation = k.relaxation;
   a.bind_ptr = c.bind_ptr.p;
@@ -771,15 +792,22 @@ static TailArgs tail_args(Context& c, const FrameConst& k) {
   return a;
 }
 
+// Lists ahead of the wait while all vertices are in flight at once.
+template <bool TAPE, bool AHEAD>
+static void stage(Context& c, const TailArgs& a, bool lra, bool contacts) {
+  auto kern = lra ? (contacts ? k_stage<true, true, TAPE, AHEAD> : k_stage<true, false, TAPE, AHEAD>)
+                  : k_stage<false, true, TAPE, AHEAD>;
+  launch_k(c.pdl, kern, grid_for(c.nv, c.vertex_block), c.vertex_block, 0, c.stream, a);
+}
 void launch_stage(Context& c, const FrameConst& k, bool lra, bool contacts, float4* tape) {
   if (!lra && !contacts) return;
-  auto kern = tape ? (lra ? (contacts ? k_stage<true, true, true> : k_stage<true, false, true>)
-                          : k_stage<false, true, true>)
-                   : (lra ? (contacts ? k_stage<true, true, false> : k_stage<true, false, false>)
-                          : k_stage<false, true, false>);
   TailArgs a = tail_args(c, k);
   a.tape = tape;
-  launch_k(c.pdl, kern, grid_for(c.nv, c.vertex_block), c.vertex_block, 0, c.stream, a);
+  const bool ahead = c.nv <= 640u * (uint32_t)c.num_sms;
+  if (tape)
+    ahead ? stage<true, true>(c, a, lra, contacts) : stage<true, false>(c, a, lra, contacts);
+  else
+    ahead ? stage<false, true>(c, a, lra, contacts) : stage<false, false>(c, a, lra, contacts);
 }
 
 void launch_ee(Context& c, const FrameConst& k, bool contacts, bool bindings, float4* tape,
