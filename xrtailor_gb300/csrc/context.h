@@ -219,6 +219,7 @@ struct DiffState {
   bool s_tiled = false, b_tiled = false;
   bool s_stage = false, b_stage = false;  // tiled reverse stages each tile's tape in shared memory
   uint32_t s_block = 256, b_block = 256;  // threads per tile block of the tiled reverse
+  bool s_pair = false, b_pair = false;    // ... two groups of as many
   DBuf<float4> t_sx;                    // S x I x E x 2: stretch inputs (x with inverse mass)
   DBuf<float> t_sl;                     // S x I x E: stretch multipliers in
   DBuf<float4> t_bx;                    // S x I x B x 4: bend inputs

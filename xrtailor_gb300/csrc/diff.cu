@@ -101,43 +101,62 @@ __device__ __forceinline__ void cross_bwd(f3 a, f3 b, f3 cb, f3& ab, f3& bb) {
 // exactly as the forward computes it.
 __device__ __forceinline__ float frcp(float x) { return __fdividef(1.0f, x); }
 
-// XPBD distance (stretch_project): inputs (a, b, lambda), outputs (a', b', lambda').  ga, gb hold
-// the outputs' adjoints on entry (xyz; w accumulates the inverse-mass adjoint) and the inputs'
-// on exit; lbo is lambda'-bar.  Returns false for an inactive projection (the identity: nothing
-// changes, lambda-bar = lbo); else sets lam_in_bar and adds the compliance adjoint to cbar.
+// XPBD distance (stretch_project): inputs (a, b, lambda), outputs (a', b', lambda').  forward()
+// recomputes the projection and returns whether it ran; it needs no adjoint, so the tiled reverse
+// can be ahead with it.  reverse(): ga, gb hold the outputs' adjoints on entry (xyz; w accumulates
+// the inverse-mass adjoint) and the inputs' on exit; lbo is lambda'-bar; sets lam_in_bar and adds
+// the compliance adjoint to cbar.  Where the projection did not run it is the identity: nothing
+// changes, lambda-bar = lbo.
+struct StretchVjp {
+  f3 d, n;
+  float dist, wa, wb, re, idt2, at, rD, dl, lam;
+  __device__ __forceinline__ bool forward(float4 A, float4 B, float lambda, float rest, float comp,
+                                          float dt) {
+    d = mk3(A) - mk3(B);
+    const float dd = fdot(d, d);
+    dist = sqrt_rn(dd);  // as the forward: it decides whether the projection ran
+    if (!in_range(dd)) dist = sqrtf(dd);
+    wa = A.w;
+    wb = B.w;
+    lam = lambda;
+    re = frcp(dist + kEps);
+    n = d * re;
+    idt2 = frcp(dt * dt);
+    at = comp * idt2;
+    const float C = dist - rest;
+    rD = frcp(wa + wb + at);
+    dl = (-C - at * lam) * rD;
+    return dist != rest && wa + wb > 0.0f;
+  }
+  __device__ __forceinline__ void reverse(float lbo, float4& ga, float4& gb, float& lam_in_bar,
+                                          float& cbar) const {
+    const f3 corr = dl * n;
+    // x_a' = x_a + w_a corr, x_b' = x_b - w_b corr, lambda' = lambda + dl
+    const f3 corr_bar = wa * mk3(ga) - wb * mk3(gb);
+    float wa_bar = dot(corr, mk3(ga));
+    float wb_bar = -dot(corr, mk3(gb));
+    const float dl_bar = dot(corr_bar, n) + lbo;
+    const f3 n_bar = dl * corr_bar;
+    const float N_bar = dl_bar * rD;       // dl = N / D
+    const float D_bar = -dl_bar * dl * rD;
+    const float C_bar = -N_bar;            // N = -C - at lambda
+    const float at_bar = -N_bar * lam + D_bar;
+    lam_in_bar = lbo - N_bar * at;
+    wa_bar += D_bar;
+    wb_bar += D_bar;
+    const float dist_bar = C_bar - dot(n_bar, n) * re;  // n = d / (dist + eps)
+    const f3 d_bar = n_bar * re + (dist > 0.0f ? (dist_bar * frcp(dist)) * d : mk3(0, 0, 0));
+    ga = mk4(mk3(ga) + d_bar, ga.w + wa_bar);
+    gb = mk4(mk3(gb) - d_bar, gb.w + wb_bar);
+    cbar += at_bar * idt2;
+  }
+};
 __device__ __forceinline__ bool stretch_vjp(float4 A, float4 B, float lam, float rest, float comp,
                                             float dt, float lbo, float4& ga, float4& gb,
                                             float& lam_in_bar, float& cbar) {
-  const f3 d = mk3(A) - mk3(B);
-  const float dist = sqrtf(fdot(d, d));  // as the forward: it decides whether the projection ran
-  const float wa = A.w, wb = B.w;
-  if (!(dist != rest && wa + wb > 0.0f)) return false;
-  const float re = frcp(dist + kEps);
-  const f3 n = d * re;
-  const float idt2 = frcp(dt * dt);
-  const float at = comp * idt2;
-  const float C = dist - rest;
-  const float rD = frcp(wa + wb + at);
-  const float dl = (-C - at * lam) * rD;
-  const f3 corr = dl * n;
-  // x_a' = x_a + w_a corr, x_b' = x_b - w_b corr, lambda' = lambda + dl
-  const f3 corr_bar = wa * mk3(ga) - wb * mk3(gb);
-  float wa_bar = dot(corr, mk3(ga));
-  float wb_bar = -dot(corr, mk3(gb));
-  const float dl_bar = dot(corr_bar, n) + lbo;
-  const f3 n_bar = dl * corr_bar;
-  const float N_bar = dl_bar * rD;       // dl = N / D
-  const float D_bar = -dl_bar * dl * rD;
-  const float C_bar = -N_bar;            // N = -C - at lambda
-  const float at_bar = -N_bar * lam + D_bar;
-  lam_in_bar = lbo - N_bar * at;
-  wa_bar += D_bar;
-  wb_bar += D_bar;
-  const float dist_bar = C_bar - dot(n_bar, n) * re;  // n = d / (dist + eps)
-  const f3 d_bar = n_bar * re + (dist > 0.0f ? (dist_bar * frcp(dist)) * d : mk3(0, 0, 0));
-  ga = mk4(mk3(ga) + d_bar, ga.w + wa_bar);
-  gb = mk4(mk3(gb) - d_bar, gb.w + wb_bar);
-  cbar += at_bar * idt2;
+  StretchVjp v;
+  if (!v.forward(A, B, lam, rest, comp, dt)) return false;
+  v.reverse(lbo, ga, gb, lam_in_bar, cbar);
   return true;
 }
 
@@ -182,107 +201,139 @@ __device__ __forceinline__ float acos_as_deriv(float x) {
   return (1.0f - x) * rs * dp - 0.5f * p * rs;
 }
 
-// Dihedral bend: inputs x1..x4 (w in .w), outputs x_i' = x_i + w_i lambda q_i.
-// G1..G4 hold the outputs' adjoints on entry and the inputs' on exit; returns false for an
-// inactive projection (the identity), else adds the compliance adjoint to cbar.
+// Dihedral bend: inputs x1..x4 (w in .w), outputs x_i' = x_i + w_i lambda q_i.  forward()
+// recomputes the projection from the taped inputs and returns whether it ran (else it is the
+// identity); reverse(): G1..G4 hold the outputs' adjoints on entry and the inputs' on exit, the
+// compliance adjoint is added to cbar.
+struct BendVjp {
+  f3 p2, p3, p4, n1, n2, B3, B4, B23, B24, A23, A24, q1, q2, q3, q4;
+  float w1, w2, w3, w4, theta, i23, i24, draw, d, angle, r23, r24, idt2, rs, s, rden, lam;
+  __device__ __forceinline__ bool forward(float4 A1, float4 A2, float4 A3, float4 A4, float rest,
+                                          float comp, float dt) {
+    w1 = A1.w;
+    w2 = A2.w;
+    w3 = A3.w;
+    w4 = A4.w;
+    theta = rest;
+    const f3 p1 = mk3(A1);
+    p2 = mk3(A2) - p1;
+    p3 = mk3(A3) - p1;
+    p4 = mk3(A4) - p1;
+    const f3 c23 = fcross(p2, p3), c24 = fcross(p2, p4);  // the forward's fused forms, exactly
+    const float d23 = fdot(c23, c23), d24 = fdot(c24, c24);
+    i23 = recip(sqrt_rn(d23));  // normalize's, exactly
+    i24 = recip(sqrt_rn(d24));
+    if (!(in_range(d23) && in_range(d24))) {
+      i23 = 1.0f / sqrtf(d23);
+      i24 = 1.0f / sqrtf(d24);
+    }
+    n1 = c23 * i23;
+    n2 = c24 * i24;
+    draw = fdot(n1, n2);
+    d = tclamp(draw, 0.0f, 1.0f);
+    angle = d < 1.0f ? sqrt_rn(1.0f - d) * acos_poly(d) : 0.0f;  // acos_as
+    bool ran = !(angle < kEps);  // else not projected: identity (d NaN: angle 0)
+    const float L23 = d23 * i23, L24 = d24 * i24;  // |c23|, |c24|
+    r23 = frcp(L23 + kEps);
+    r24 = frcp(L24 + kEps);
+    B3 = cross(n1, p2);
+    B4 = cross(n2, p2);
+    B23 = cross(n1, p3);
+    B24 = cross(n2, p4);
+    const f3 A3v = cross(p2, n2) + B3 * d;
+    const f3 A4v = cross(p2, n1) + B4 * d;
+    A23 = cross(p3, n2) + B23 * d;
+    A24 = cross(p4, n1) + B24 * d;
+    q3 = A3v * r23;
+    q4 = A4v * r24;
+    q2 = -(A23 * r23) - A24 * r24;
+    q1 = -q2 - q3 - q4;
+    idt2 = frcp(dt * dt);
+    const float at = comp * idt2;
+    const float denom = at + (w1 * dot(q1, q1) + w2 * dot(q2, q2) + w3 * dot(q3, q3) +
+                              w4 * dot(q4, q4));
+    if (denom < kEps) ran = false;
+    const float om = 1.0f - d * d;  // > 0: d < 1 wherever the angle passed
+    rs = rsqrtf(om);
+    s = om * rs;
+    rden = frcp(denom);
+    lam = s * (angle - theta) * rden;
+    return ran;
+  }
+  __device__ __forceinline__ void reverse(float4& G1, float4& G2, float4& G3, float4& G4,
+                                          float& cbar) const {
+    const f3 g1 = mk3(G1), g2 = mk3(G2), g3 = mk3(G3), g4 = mk3(G4);
+    // c_i = w_i lam q_i
+    const float lam_bar = w1 * dot(g1, q1) + w2 * dot(g2, q2) + w3 * dot(g3, q3) + w4 * dot(g4, q4);
+    f3 q1b = (w1 * lam) * g1, q2b = (w2 * lam) * g2, q3b = (w3 * lam) * g3, q4b = (w4 * lam) * g4;
+    float w1b = lam * dot(g1, q1), w2b = lam * dot(g2, q2), w3b = lam * dot(g3, q3),
+          w4b = lam * dot(g4, q4);
+    // lam = s (angle - theta) / denom
+    const float s_bar = lam_bar * (angle - theta) * rden;
+    const float angle_bar = lam_bar * s * rden;
+    const float denom_bar = -lam_bar * lam * rden;
+    // denom = at + sum w_i |q_i|^2
+    q1b = q1b + (2.0f * denom_bar * w1) * q1;
+    q2b = q2b + (2.0f * denom_bar * w2) * q2;
+    q3b = q3b + (2.0f * denom_bar * w3) * q3;
+    q4b = q4b + (2.0f * denom_bar * w4) * q4;
+    w1b += denom_bar * dot(q1, q1);
+    w2b += denom_bar * dot(q2, q2);
+    w3b += denom_bar * dot(q3, q3);
+    w4b += denom_bar * dot(q4, q4);
+    cbar += denom_bar * idt2;
+    // q1 = -q2 - q3 - q4
+    q2b = q2b - q1b;
+    q3b = q3b - q1b;
+    q4b = q4b - q1b;
+    // q3 = A3v / e23, q4 = A4v / e24, q2 = -A23 / e23 - A24 / e24  (e = |c| + eps)
+    const f3 A3b = q3b * r23, A4b = q4b * r24, A23b = -(q2b * r23), A24b = -(q2b * r24);
+    const float e23b = (-dot(q3b, q3) + dot(q2b, A23) * r23) * r23;
+    const float e24b = (-dot(q4b, q4) + dot(q2b, A24) * r24) * r24;
+    f3 p2b = mk3(0, 0, 0), p3b = mk3(0, 0, 0), p4b = mk3(0, 0, 0);
+    f3 n1b = mk3(0, 0, 0), n2b = mk3(0, 0, 0);
+    float db = 0.0f;
+    // A3v = p2 x n2 + (n1 x p2) d
+    cross_bwd(p2, n2, A3b, p2b, n2b);
+    cross_bwd(n1, p2, A3b * d, n1b, p2b);
+    db += dot(A3b, B3);
+    // A4v = p2 x n1 + (n2 x p2) d
+    cross_bwd(p2, n1, A4b, p2b, n1b);
+    cross_bwd(n2, p2, A4b * d, n2b, p2b);
+    db += dot(A4b, B4);
+    // A23 = p3 x n2 + (n1 x p3) d
+    cross_bwd(p3, n2, A23b, p3b, n2b);
+    cross_bwd(n1, p3, A23b * d, n1b, p3b);
+    db += dot(A23b, B23);
+    // A24 = p4 x n1 + (n2 x p4) d
+    cross_bwd(p4, n1, A24b, p4b, n1b);
+    cross_bwd(n2, p4, A24b * d, n2b, p4b);
+    db += dot(A24b, B24);
+    // s = sqrt(1 - d^2); angle = acos_as(d)
+    db += s_bar * (-d * rs) + angle_bar * acos_as_deriv(d);
+    // d = clamp(n1 . n2, 0, 1)
+    if (draw > 0.0f && draw < 1.0f) {
+      n1b = n1b + db * n2;
+      n2b = n2b + db * n1;
+    }
+    // n = c / |c|, e = |c| + eps
+    const f3 c23b = (n1b - dot(n1, n1b) * n1) * i23 + e23b * n1;
+    const f3 c24b = (n2b - dot(n2, n2b) * n2) * i24 + e24b * n2;
+    cross_bwd(p2, p3, c23b, p2b, p3b);
+    cross_bwd(p2, p4, c24b, p2b, p4b);
+    const f3 p1b = -(p2b + p3b + p4b);
+    G1 = mk4(g1 + p1b, G1.w + w1b);
+    G2 = mk4(g2 + p2b, G2.w + w2b);
+    G3 = mk4(g3 + p3b, G3.w + w3b);
+    G4 = mk4(g4 + p4b, G4.w + w4b);
+  }
+};
 __device__ __forceinline__ bool bend_vjp(float4 A1, float4 A2, float4 A3, float4 A4, float theta,
                                          float comp, float dt, float4& G1, float4& G2, float4& G3,
                                          float4& G4, float& cbar) {
-  const float w1 = A1.w, w2 = A2.w, w3 = A3.w, w4 = A4.w;
-  const f3 p1 = mk3(A1);
-  const f3 p2 = mk3(A2) - p1, p3 = mk3(A3) - p1, p4 = mk3(A4) - p1;
-  const f3 c23 = fcross(p2, p3), c24 = fcross(p2, p4);  // the forward's fused forms, exactly
-  const float d23 = fdot(c23, c23), d24 = fdot(c24, c24);
-  const float i23 = 1.0f / sqrtf(d23), i24 = 1.0f / sqrtf(d24);  // normalize's, exactly
-  const f3 n1 = c23 * i23, n2 = c24 * i24;
-  const float draw = fdot(n1, n2);
-  const float d = tclamp(draw, 0.0f, 1.0f);
-  const float angle = acos_as(d);
-  if (angle < kEps || isnan(d)) return false;  // not projected: identity
-  const float L23 = d23 * i23, L24 = d24 * i24;  // |c23|, |c24|
-  const float r23 = frcp(L23 + kEps), r24 = frcp(L24 + kEps);
-  const f3 B3 = cross(n1, p2), B4 = cross(n2, p2), B23 = cross(n1, p3), B24 = cross(n2, p4);
-  const f3 A3v = cross(p2, n2) + B3 * d;
-  const f3 A4v = cross(p2, n1) + B4 * d;
-  const f3 A23 = cross(p3, n2) + B23 * d;
-  const f3 A24 = cross(p4, n1) + B24 * d;
-  const f3 q3 = A3v * r23, q4 = A4v * r24;
-  const f3 q2 = -(A23 * r23) - A24 * r24;
-  const f3 q1 = -q2 - q3 - q4;
-  const float idt2 = frcp(dt * dt);
-  const float at = comp * idt2;
-  const float denom = at + (w1 * dot(q1, q1) + w2 * dot(q2, q2) + w3 * dot(q3, q3) +
-                            w4 * dot(q4, q4));
-  if (denom < kEps) return false;
-  const float om = 1.0f - d * d;  // > 0: d < 1 wherever the angle passed
-  const float rs = rsqrtf(om);
-  const float s = om * rs;
-  const float rden = frcp(denom);
-  const float lam = s * (angle - theta) * rden;
-  const f3 g1 = mk3(G1), g2 = mk3(G2), g3 = mk3(G3), g4 = mk3(G4);
-  // c_i = w_i lam q_i
-  const float lam_bar = w1 * dot(g1, q1) + w2 * dot(g2, q2) + w3 * dot(g3, q3) + w4 * dot(g4, q4);
-  f3 q1b = (w1 * lam) * g1, q2b = (w2 * lam) * g2, q3b = (w3 * lam) * g3, q4b = (w4 * lam) * g4;
-  float w1b = lam * dot(g1, q1), w2b = lam * dot(g2, q2), w3b = lam * dot(g3, q3),
-        w4b = lam * dot(g4, q4);
-  // lam = s (angle - theta) / denom
-  const float s_bar = lam_bar * (angle - theta) * rden;
-  const float angle_bar = lam_bar * s * rden;
-  const float denom_bar = -lam_bar * lam * rden;
-  // denom = at + sum w_i |q_i|^2
-  q1b = q1b + (2.0f * denom_bar * w1) * q1;
-  q2b = q2b + (2.0f * denom_bar * w2) * q2;
-  q3b = q3b + (2.0f * denom_bar * w3) * q3;
-  q4b = q4b + (2.0f * denom_bar * w4) * q4;
-  w1b += denom_bar * dot(q1, q1);
-  w2b += denom_bar * dot(q2, q2);
-  w3b += denom_bar * dot(q3, q3);
-  w4b += denom_bar * dot(q4, q4);
-  cbar += denom_bar * idt2;
-  // q1 = -q2 - q3 - q4
-  q2b = q2b - q1b;
-  q3b = q3b - q1b;
-  q4b = q4b - q1b;
-  // q3 = A3v / e23, q4 = A4v / e24, q2 = -A23 / e23 - A24 / e24  (e = |c| + eps)
-  const f3 A3b = q3b * r23, A4b = q4b * r24, A23b = -(q2b * r23), A24b = -(q2b * r24);
-  const float e23b = (-dot(q3b, q3) + dot(q2b, A23) * r23) * r23;
-  const float e24b = (-dot(q4b, q4) + dot(q2b, A24) * r24) * r24;
-  f3 p2b = mk3(0, 0, 0), p3b = mk3(0, 0, 0), p4b = mk3(0, 0, 0);
-  f3 n1b = mk3(0, 0, 0), n2b = mk3(0, 0, 0);
-  float db = 0.0f;
-  // A3v = p2 x n2 + (n1 x p2) d
-  cross_bwd(p2, n2, A3b, p2b, n2b);
-  cross_bwd(n1, p2, A3b * d, n1b, p2b);
-  db += dot(A3b, B3);
-  // A4v = p2 x n1 + (n2 x p2) d
-  cross_bwd(p2, n1, A4b, p2b, n1b);
-  cross_bwd(n2, p2, A4b * d, n2b, p2b);
-  db += dot(A4b, B4);
-  // A23 = p3 x n2 + (n1 x p3) d
-  cross_bwd(p3, n2, A23b, p3b, n2b);
-  cross_bwd(n1, p3, A23b * d, n1b, p3b);
-  db += dot(A23b, B23);
-  // A24 = p4 x n1 + (n2 x p4) d
-  cross_bwd(p4, n1, A24b, p4b, n1b);
-  cross_bwd(n2, p4, A24b * d, n2b, p4b);
-  db += dot(A24b, B24);
-  // s = sqrt(1 - d^2); angle = acos_as(d)
-  db += s_bar * (-d * rs) + angle_bar * acos_as_deriv(d);
-  // d = clamp(n1 . n2, 0, 1)
-  if (draw > 0.0f && draw < 1.0f) {
-    n1b = n1b + db * n2;
-    n2b = n2b + db * n1;
-  }
-  // n = c / |c|, e = |c| + eps
-  const f3 c23b = (n1b - dot(n1, n1b) * n1) * i23 + e23b * n1;
-  const f3 c24b = (n2b - dot(n2, n2b) * n2) * i24 + e24b * n2;
-  cross_bwd(p2, p3, c23b, p2b, p3b);
-  cross_bwd(p2, p4, c24b, p2b, p4b);
-  const f3 p1b = -(p2b + p3b + p4b);
-  G1 = mk4(g1 + p1b, G1.w + w1b);
-  G2 = mk4(g2 + p2b, G2.w + w2b);
-  G3 = mk4(g3 + p3b, G3.w + w3b);
-  G4 = mk4(g4 + p4b, G4.w + w4b);
+  BendVjp v;
+  if (!v.forward(A1, A2, A3, A4, theta, comp, dt)) return false;
+  v.reverse(G1, G2, G3, G4, cbar);
   return true;
 }
 
@@ -321,16 +372,72 @@ __global__ void k_bend_bwd(const uint32_t* __restrict__ order, uint32_t begin, u
 // (stretch, 4 B) or rest angle and compliance (bend, 8 B) per constraint; num_local + 1
 // offsets.
 
+// One 16-byte copy to shared memory that no register waits for; copy_wait() ends all of a thread's.
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The local colors of a tile, last to first: forward(j, v) recomputes element j, one(j, ran, v) runs
+// its reverse.  The elements of a color beyond the first NT run both in the reverse's turn.
+template <int NT, bool PAIR, class Vjp, class Forward, class One>
+__device__ __forceinline__ void reverse_colors(const uint32_t* so, int num_local, Forward forward,
+                                               One one) {
+  const uint32_t tid = threadIdx.x % NT;
+  Vjp v;
+  if (!PAIR) {
+    for (int l = num_local - 1; l >= 0; --l) {
+      for (uint32_t j = so[l] + tid; j < so[l + 1]; j += NT) {
+        const bool ran = forward(j, v);
+        one(j, ran, v);
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  const int group = (int)(threadIdx.x / NT);
+  bool ran = false;
+  auto ahead = [&](int l) {
+    if (l >= 0 && so[l] + tid < so[l + 1]) ran = forward(so[l] + tid, v);
+  };
+  if (((num_local - 1) & 1) == group) ahead(num_local - 1);
+  for (int l = num_local - 1; l >= 0; --l) {
+    if ((l & 1) == group) {
+      uint32_t j = so[l] + tid;
+      if (j < so[l + 1]) one(j, ran, v);
+      for (j += NT; j < so[l + 1]; j += NT) {
+        ran = forward(j, v);
+        one(j, ran, v);
+      }
+    } else {
+      ahead(l - 1);
+    }
+    __syncthreads();
+  }
+}
+
+// PAIR: two groups of NT threads take the local colors in turn; while one runs a color's reverse, the
+// other runs the projections of the next color forward, which need only the tape.  A launch is bound
+// by its chain of local colors, each a barrier and an element's arithmetic in one thread: 108 tiles
+// of six 96 x 96 cloths take 25.6 (bend) and 16.7 us (stretch) with one group and a compliance
+// adjoint added in global memory per color, 18.2 and 12.9 with two groups and the sums parked beside
+// the record, 16.9 and 10.7 with the tape copied asynchronously.  Releasing the next launch at the
+// start instead of the end: the same launches, but the frames 91 ms against 83.
+//
 // STAGE: the tile's slice of the tape (contiguous slots c0 .. c0 + nc) is loaded into shared
 // memory up front, all loads in flight at once, instead of one dependent global load per local
 // color step; for tiles whose slice does not fit, the reverse reads the tape in place.
-template <bool RESET, int NT, bool STAGE>
-__global__ void __launch_bounds__(NT) k_stretch_tiles_bwd(
+template <bool RESET, int NT, bool STAGE, bool PAIR>
+__global__ void __launch_bounds__(PAIR ? 2 * NT : NT) k_stretch_tiles_bwd(
     const int4* __restrict__ con, const uint32_t* __restrict__ foot,
     const int4* __restrict__ meta, const uint32_t* __restrict__ lofs, uint32_t tile_begin,
     uint32_t num_local, uint32_t max_foot, uint32_t max_cons, float dt,
     const float4* __restrict__ tx, const float* __restrict__ tl, float4* __restrict__ G,
     float* __restrict__ lam_bar, float* __restrict__ comp_bar) {
+  constexpr int kThreads = PAIR ? 2 * NT : NT;
   extern __shared__ float4 smem[];
   float4* sg = smem;
   float4* stx = sg + max_foot;                               // STAGE: 2 x max_cons
@@ -339,50 +446,57 @@ __global__ void __launch_bounds__(NT) k_stretch_tiles_bwd(
   float* stl = slb + max_cons;                               // STAGE: max_cons
   uint32_t* so = reinterpret_cast<uint32_t*>(stl + (STAGE ? max_cons : 0));
   uint32_t* sf = so + num_local + 1;
-  const TileFrame f = tile_prologue<NT>(foot, meta, lofs, tile_begin + blockIdx.x, num_local, so);
+  const TileFrame f =
+      tile_prologue<kThreads>(foot, meta, lofs, tile_begin + blockIdx.x, num_local, so);
   const uint32_t c0 = (uint32_t)f.m.z, nc = (uint32_t)f.m.w;
-  for (uint32_t j = threadIdx.x; j < nc; j += NT) sc[j] = __ldg(&con[c0 + j]);  // setup data
+  for (uint32_t j = threadIdx.x; j < nc; j += kThreads) copy16(&sc[j], &con[c0 + j]);  // setup data
   pdl_wait();  // the tape and the adjoints are written by earlier launches of the reverse
   if (STAGE) {
     const float4* src = tx + 2 * (size_t)c0;
-    for (uint32_t k = threadIdx.x; k < 2 * nc; k += NT) stx[k] = src[k];
+    for (uint32_t k = threadIdx.x; k < 2 * nc; k += kThreads) copy16(&stx[k], &src[k]);
   }
-  for (uint32_t j = threadIdx.x; j < nc; j += NT) {
+  for (uint32_t j = threadIdx.x; j < nc; j += kThreads) {
     slb[j] = lam_bar[c0 + j];
     if (STAGE) stl[j] = tl[c0 + j];
   }
-  tile_gather<NT>(f, G, sg, sf);
+  tile_gather<kThreads>(f, G, sg, sf);
+  copy_wait();
   __syncthreads();
   const float4* ax = STAGE ? stx : tx + 2 * (size_t)c0;
   const float* al = STAGE ? stl : tl + c0;
-  for (int l = (int)num_local - 1; l >= 0; --l) {
-    const uint32_t ce = so[l + 1];
-    for (uint32_t j = so[l] + threadIdx.x; j < ce; j += NT) {
-      const int4 c = sc[j];
+  auto one = [&](uint32_t j, bool ran, const StretchVjp& v) {
+    const int4 c = sc[j];
+    float lin = slb[j], cb = 0.0f;
+    if (ran) {
       float4 ga = sg[c.x], gb = sg[c.y];
-      float lin = slb[j], cb = 0.0f;
-      if (stretch_vjp(ax[2 * j], ax[2 * j + 1], al[j], __int_as_float(c.z), __int_as_float(c.w),
-                      dt, slb[j], ga, gb, lin, cb)) {
-        sg[c.x] = ga;
-        sg[c.y] = gb;
-        comp_bar[c0 + j] += cb;
-      }
-      slb[j] = RESET ? 0.0f : lin;
+      v.reverse(slb[j], ga, gb, lin, cb);
+      sg[c.x] = ga;
+      sg[c.y] = gb;
     }
-    __syncthreads();
-  }
+    slb[j] = RESET ? 0.0f : lin;
+    sc[j].w = __float_as_int(cb);  // the compliance, read by forward() before
+  };
+  auto forward = [&](uint32_t j, StretchVjp& v) {
+    const int4 c = sc[j];
+    return v.forward(ax[2 * j], ax[2 * j + 1], al[j], __int_as_float(c.z), __int_as_float(c.w), dt);
+  };
+  reverse_colors<NT, PAIR, StretchVjp>(so, (int)num_local, forward, one);
   pdl_release();
-  tile_scatter<NT>((uint32_t)f.m.y, G, sg, sf);
-  for (uint32_t j = threadIdx.x; j < nc; j += NT) lam_bar[c0 + j] = slb[j];
+  tile_scatter<kThreads>((uint32_t)f.m.y, G, sg, sf);
+  for (uint32_t j = threadIdx.x; j < nc; j += kThreads) {
+    lam_bar[c0 + j] = slb[j];
+    comp_bar[c0 + j] += __int_as_float(sc[j].w);
+  }
 }
 
-template <int NT, bool STAGE>
-__global__ void __launch_bounds__(NT) k_bend_tiles_bwd(
+template <int NT, bool STAGE, bool PAIR>
+__global__ void __launch_bounds__(PAIR ? 2 * NT : NT) k_bend_tiles_bwd(
     const int4* __restrict__ idx, const float2* __restrict__ tc,
     const uint32_t* __restrict__ foot, const int4* __restrict__ meta,
     const uint32_t* __restrict__ lofs, uint32_t tile_begin, uint32_t num_local,
     uint32_t max_foot, uint32_t max_cons, float dt, const float4* __restrict__ tx,
     float4* __restrict__ G, float* __restrict__ bcomp_bar) {
+  constexpr int kThreads = PAIR ? 2 * NT : NT;
   extern __shared__ float4 smem[];
   float4* sg = smem;
   float4* stx = sg + max_foot;                               // STAGE: 4 x max_cons
@@ -390,40 +504,44 @@ __global__ void __launch_bounds__(NT) k_bend_tiles_bwd(
   float2* st = reinterpret_cast<float2*>(sc + max_cons);
   uint32_t* so = reinterpret_cast<uint32_t*>(st + max_cons);
   uint32_t* sf = so + num_local + 1;
-  const TileFrame f = tile_prologue<NT>(foot, meta, lofs, tile_begin + blockIdx.x, num_local, so);
+  const TileFrame f =
+      tile_prologue<kThreads>(foot, meta, lofs, tile_begin + blockIdx.x, num_local, so);
   const uint32_t c0 = (uint32_t)f.m.z, nc = (uint32_t)f.m.w;
-  for (uint32_t j = threadIdx.x; j < nc; j += NT) {  // setup data
-    sc[j] = __ldg(&idx[c0 + j]);
+  for (uint32_t j = threadIdx.x; j < nc; j += kThreads) {  // setup data
+    copy16(&sc[j], &idx[c0 + j]);
     st[j] = __ldg(&tc[c0 + j]);
   }
   pdl_wait();  // the tape and the adjoints are written by earlier launches of the reverse
   if (STAGE) {
     const float4* src = tx + 4 * (size_t)c0;
-    for (uint32_t k = threadIdx.x; k < 4 * nc; k += NT) stx[k] = src[k];
+    for (uint32_t k = threadIdx.x; k < 4 * nc; k += kThreads) copy16(&stx[k], &src[k]);
   }
-  tile_gather<NT>(f, G, sg, sf);
+  tile_gather<kThreads>(f, G, sg, sf);
+  copy_wait();
   __syncthreads();
   const float4* ax = STAGE ? stx : tx + 4 * (size_t)c0;
-  for (int l = (int)num_local - 1; l >= 0; --l) {
-    const uint32_t ce = so[l + 1];
-    for (uint32_t j = so[l] + threadIdx.x; j < ce; j += NT) {
+  auto one = [&](uint32_t j, bool ran, const BendVjp& v) {
+    float cb = 0.0f;
+    if (ran) {
       const int4 b = sc[j];
-      const float2 th = st[j];
-      const float4* s = ax + 4 * (size_t)j;
       float4 G1 = sg[b.x], G2 = sg[b.y], G3 = sg[b.z], G4 = sg[b.w];
-      float cb = 0.0f;
-      if (bend_vjp(s[0], s[1], s[2], s[3], th.x, th.y, dt, G1, G2, G3, G4, cb)) {
-        sg[b.x] = G1;
-        sg[b.y] = G2;
-        sg[b.z] = G3;
-        sg[b.w] = G4;
-        bcomp_bar[c0 + j] += cb;
-      }
+      v.reverse(G1, G2, G3, G4, cb);
+      sg[b.x] = G1;
+      sg[b.y] = G2;
+      sg[b.z] = G3;
+      sg[b.w] = G4;
     }
-    __syncthreads();
-  }
+    st[j].x = cb;  // the rest angle, read by forward() before
+  };
+  auto forward = [&](uint32_t j, BendVjp& v) {
+    const float2 th = st[j];
+    const float4* s = ax + 4 * (size_t)j;
+    return v.forward(s[0], s[1], s[2], s[3], th.x, th.y, dt);
+  };
+  reverse_colors<NT, PAIR, BendVjp>(so, (int)num_local, forward, one);
   pdl_release();
-  tile_scatter<NT>((uint32_t)f.m.y, G, sg, sf);
+  tile_scatter<kThreads>((uint32_t)f.m.y, G, sg, sf);
+  for (uint32_t j = threadIdx.x; j < nc; j += kThreads) bcomp_bar[c0 + j] += st[j].x;
 }
 
 // LRA (all slots pinned) + VF-CCD + VF-DCD, per vertex, Jacobi (Gin -> Gout).  The slot sources'
@@ -677,61 +795,69 @@ using BendBwdKernel = void (*)(const int4*, const float2*, const uint32_t*, cons
                                const uint32_t*, uint32_t, uint32_t, uint32_t, uint32_t, float,
                                const float4*, float4*, float*);
 
-template <int NT>
+template <int NT, bool PAIR>
 StretchBwdKernel stretch_bwd_nt(bool reset, bool stage) {
-  return reset ? (stage ? k_stretch_tiles_bwd<true, NT, true> : k_stretch_tiles_bwd<true, NT, false>)
-               : (stage ? k_stretch_tiles_bwd<false, NT, true>
-                        : k_stretch_tiles_bwd<false, NT, false>);
+  return reset ? (stage ? k_stretch_tiles_bwd<true, NT, true, PAIR>
+                        : k_stretch_tiles_bwd<true, NT, false, PAIR>)
+               : (stage ? k_stretch_tiles_bwd<false, NT, true, PAIR>
+                        : k_stretch_tiles_bwd<false, NT, false, PAIR>);
 }
-StretchBwdKernel stretch_bwd_kernel(uint32_t block, bool reset, bool stage) {
-  return block == 128 ? stretch_bwd_nt<128>(reset, stage)
-         : block == 256 ? stretch_bwd_nt<256>(reset, stage)
-                        : stretch_bwd_nt<512>(reset, stage);
+// `pair`: 2 x 128 threads (block 128 only).
+StretchBwdKernel stretch_bwd_kernel(uint32_t block, bool reset, bool stage, bool pair) {
+  return pair           ? stretch_bwd_nt<128, true>(reset, stage)
+         : block == 128 ? stretch_bwd_nt<128, false>(reset, stage)
+         : block == 256 ? stretch_bwd_nt<256, false>(reset, stage)
+                        : stretch_bwd_nt<512, false>(reset, stage);
 }
 StretchBwdKernel stretch_bwd_kernel(const Context& c, bool reset) {
-  return stretch_bwd_kernel(c.diff.s_block, reset, c.diff.s_stage);
+  return stretch_bwd_kernel(c.diff.s_block, reset, c.diff.s_stage, c.diff.s_pair);
 }
-template <int NT>
+template <int NT, bool PAIR>
 BendBwdKernel bend_bwd_nt(bool stage) {
-  return stage ? k_bend_tiles_bwd<NT, true> : k_bend_tiles_bwd<NT, false>;
+  return stage ? k_bend_tiles_bwd<NT, true, PAIR> : k_bend_tiles_bwd<NT, false, PAIR>;
 }
-BendBwdKernel bend_bwd_kernel(uint32_t block, bool stage) {
-  return block == 128 ? bend_bwd_nt<128>(stage)
-         : block == 256 ? bend_bwd_nt<256>(stage)
-                        : bend_bwd_nt<512>(stage);
+BendBwdKernel bend_bwd_kernel(uint32_t block, bool stage, bool pair) {
+  return pair           ? bend_bwd_nt<128, true>(stage)
+         : block == 128 ? bend_bwd_nt<128, false>(stage)
+         : block == 256 ? bend_bwd_nt<256, false>(stage)
+                        : bend_bwd_nt<512, false>(stage);
 }
 BendBwdKernel bend_bwd_kernel(const Context& c) {
-  return bend_bwd_kernel(c.diff.b_block, c.diff.b_stage);
+  return bend_bwd_kernel(c.diff.b_block, c.diff.b_stage, c.diff.b_pair);
 }
 
 // Launch shape of a tiled reverse: 128-thread blocks where the footprints fit (a local color of
 // a tile rarely has more elements, and four blocks per SM hold more tiles at once), else the
 // forward's; the tape slice is staged when the staged blocks still hold the largest tile color
-// in one wave (or lose no resident blocks), read in place otherwise.
+// in one wave (or lose no resident blocks), read in place otherwise.  Paired groups where a tile
+// color leaves each SM one block at most: with more, the blocks fill each other's gaps.
 template <typename K>
-cudaError_t choose_reverse_shape(const Context& c, const TiledSet& T, K (*kernel)(uint32_t, bool),
+cudaError_t choose_reverse_shape(const Context& c, const TiledSet& T, K (*kernel)(uint32_t, bool, bool),
                                  size_t smem_plain, size_t smem_staged, int smem_max,
-                                 uint32_t& block, bool& stage) {
+                                 uint32_t& block, bool& stage, bool& pair) {
   block = T.max_foot <= kFootPerThread * 128u ? 128u : T.block;
   uint32_t widest = 0;
   for (const ColorRange& r : T.tile_colors) widest = std::max(widest, r.end - r.begin);
   int occ_plain = 0, occ_staged = 0;
-  cudaError_t e = raise_smem((const void*)kernel(block, false), smem_plain);
+  cudaError_t e = raise_smem((const void*)kernel(block, false, false), smem_plain);
   if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_plain, kernel(block, false),
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_plain, kernel(block, false, false),
                                                       (int)block, smem_plain);
   if (e != cudaSuccess) return e;
   stage = false;
   if (smem_staged <= (size_t)smem_max) {
-    e = raise_smem((const void*)kernel(block, true), smem_staged);
+    e = raise_smem((const void*)kernel(block, true, false), smem_staged);
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_staged, kernel(block, true),
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_staged, kernel(block, true, false),
                                                         (int)block, smem_staged);
     if (e != cudaSuccess) return e;
     stage = occ_staged > 0 && ((uint64_t)occ_staged * (uint64_t)c.num_sms >= widest ||
                                occ_staged >= occ_plain);
   }
-  return cudaSuccess;
+  pair = block == 128 && widest <= (uint32_t)c.num_sms;
+  return pair ? raise_smem((const void*)kernel(block, stage, true),
+                           stage ? smem_staged : smem_plain)
+              : cudaSuccess;
 }
 
 cudaError_t configure_tiled_adjoint(Context& c, int smem_max) {
@@ -744,16 +870,18 @@ cudaError_t configure_tiled_adjoint(Context& c, int smem_max) {
     const TiledSet& T = c.s_tiles;
     if (e == cudaSuccess)
       e = choose_reverse_shape(
-          c, T, +[](uint32_t b, bool s) { return stretch_bwd_kernel(b, false, s); },
-          stretch_bwd_smem(T, false), stretch_bwd_smem(T, true), smem_max, D.s_block, D.s_stage);
+          c, T, +[](uint32_t b, bool s, bool p) { return stretch_bwd_kernel(b, false, s, p); },
+          stretch_bwd_smem(T, false), stretch_bwd_smem(T, true), smem_max, D.s_block, D.s_stage,
+          D.s_pair);
     set((const void*)stretch_bwd_kernel(c, true), stretch_bwd_smem(c));
   }
   if (D.b_tiled) {
     const TiledSet& T = c.b_tiles;
     if (e == cudaSuccess)
       e = choose_reverse_shape(
-          c, T, +[](uint32_t b, bool s) { return bend_bwd_kernel(b, s); },
-          bend_bwd_smem(T, false), bend_bwd_smem(T, true), smem_max, D.b_block, D.b_stage);
+          c, T, +[](uint32_t b, bool s, bool p) { return bend_bwd_kernel(b, s, p); },
+          bend_bwd_smem(T, false), bend_bwd_smem(T, true), smem_max, D.b_block, D.b_stage,
+          D.b_pair);
   }
   return e;
 }
@@ -769,7 +897,7 @@ void stretch_tiles_bwd(Context& c, float dt, bool reset, size_t ti) {
   for (int k = (int)T.tile_colors.size() - 1; k >= 0; --k) {
     const ColorRange r = T.tile_colors[k];
     if (r.end > r.begin)
-      launch_k(c.pdl, kern, r.end - r.begin, D.s_block, smem, c.stream, c.s_con.p, T.foot.p,
+      launch_k(c.pdl, kern, r.end - r.begin, D.s_block * (D.s_pair ? 2 : 1), smem, c.stream, c.s_con.p, T.foot.p,
                T.meta.p, T.lofs.p, r.begin, T.num_local, T.max_foot, T.max_cons, dt, tx, tl,
                D.G.p, D.lam_bar.p, D.comp_bar.p);
   }
@@ -784,7 +912,7 @@ void bend_tiles_bwd(Context& c, float dt, size_t ti) {
   for (int k = (int)T.tile_colors.size() - 1; k >= 0; --k) {
     const ColorRange r = T.tile_colors[k];
     if (r.end > r.begin)
-      launch_k(c.pdl, kern, r.end - r.begin, D.b_block, smem, c.stream, c.b_idx.p, c.b_tc.p,
+      launch_k(c.pdl, kern, r.end - r.begin, D.b_block * (D.b_pair ? 2 : 1), smem, c.stream, c.b_idx.p, c.b_tc.p,
                T.foot.p, T.meta.p, T.lofs.p, r.begin, T.num_local, T.max_foot, T.max_cons, dt,
                tx, D.G.p, D.bcomp_bar.p);
   }
