@@ -52,12 +52,13 @@ __global__ void k_cell_bounds(const uint32_t* __restrict__ skey, uint32_t nv,
   if (id == nv - 1) cell_end[h] = id + 1;
 }
 
-__global__ void k_cache_neighbors(const uint32_t* __restrict__ sidx,
-                                  const uint32_t* __restrict__ cell_start,
-                                  const uint32_t* __restrict__ cell_end,
-                                  const float4* __restrict__ x, const float4* __restrict__ x_init,
-                                  uint32_t nv, InstView I, uint32_t maxnb,
-                                  uint32_t* __restrict__ neighbors) {
+// A lane per vertex, cell by cell.
+__global__ void k_cache_neighbors_lane(const uint32_t* __restrict__ sidx,
+                                       const uint32_t* __restrict__ cell_start,
+                                       const uint32_t* __restrict__ cell_end,
+                                       const float4* __restrict__ x,
+                                       const float4* __restrict__ x_init, uint32_t nv, InstView I,
+                                       uint32_t maxnb, uint32_t* __restrict__ neighbors) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= nv) return;
   const uint32_t id = sidx[tid];
@@ -89,6 +90,67 @@ __global__ void k_cache_neighbors(const uint32_t* __restrict__ sidx,
         }
       }
   if (ni < limit) neighbors[ni] = kNone;
+}
+
+// A warp per vertex: 27 lanes look up the cells around it, the cells' entries are numbered through in
+// cell order, and 32 entries at a time are tested and appended in that order.  The same lists.
+constexpr int kCells = 27;
+__global__ void k_cache_neighbors(const uint32_t* __restrict__ sidx,
+                                  const uint32_t* __restrict__ cell_start,
+                                  const uint32_t* __restrict__ cell_end,
+                                  const float4* __restrict__ x, const float4* __restrict__ x_init,
+                                  uint32_t nv, InstView I, uint32_t maxnb,
+                                  uint32_t* __restrict__ neighbors) {
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t lane = threadIdx.x & 31u;
+  if (warp >= nv) return;
+  const uint32_t id = sidx[warp];
+  const InstanceRec r = inst_rec(I, inst_index(I, id));
+  const f3 pos = mk3(x[id]), orig = mk3(x_init[id]);
+  // cell `lane`: z runs fastest, then y
+  const int cx = (int)lane / 9, cy = (int)lane / 3 % 3, cz = (int)lane % 3;
+  uint32_t start = 0, size = 0;
+  if (lane < kCells) {
+    const uint32_t h = r.table_base +
+                       (uint32_t)hash_coords(int_coord(pos.x, r.spacing) - 1 + cx,
+                                             int_coord(pos.y, r.spacing) - 1 + cy,
+                                             int_coord(pos.z, r.spacing) - 1 + cz,
+                                             (int)r.table_size);
+    start = cell_start[h];
+    const uint32_t end = cell_end[h];
+    if (start != kNone) size = min(end, start + maxnb) - start;
+  }
+  uint32_t upto = size;  // entries of the cells up to this lane's
+#pragma unroll
+  for (int d = 1; d < 32; d *= 2) {
+    const uint32_t o = __shfl_up_sync(kAll, upto, d);
+    if (lane >= (uint32_t)d) upto += o;
+  }
+  const uint32_t total = __shfl_sync(kAll, upto, 31);
+  start -= upto - size;  // entry e of the numbering is start + e of its cell
+  uint32_t found = 0;
+  for (uint32_t base = 0; base < total && found < maxnb; base += 32) {
+    const uint32_t e = base + lane;
+    uint32_t cell = 0;  // the first cell with upto > e
+#pragma unroll
+    for (int d = 16; d > 0; d /= 2)
+      if (__shfl_sync(kAll, upto, (int)cell + d - 1) <= e) cell += d;
+    const uint32_t first = __shfl_sync(kAll, start, (int)(cell & 31u));
+    uint32_t nb = id;
+    bool near = false;
+    if (e < total) {
+      nb = sidx[first + e];
+      const f3 dp = pos - mk3(x[nb]);
+      const f3 d0 = orig - mk3(x_init[nb]);
+      near = nb != id && dot(dp, dp) < r.spacing2 && dot(d0, d0) > r.d2;
+    }
+    const unsigned m = __ballot_sync(kAll, near);
+    const uint32_t at = found + __popc(m & ((1u << lane) - 1u));
+    if (near && at < maxnb) neighbors[id + (size_t)nv * at] = nb;
+    found += __popc(m);
+  }
+  if (lane == 0 && found < maxnb) neighbors[id + (size_t)nv * found] = kNone;
 }
 
 __device__ __forceinline__ f3 friction_of(float mu, f3 correction, f3 rel_vel) {
@@ -397,9 +459,18 @@ void launch_hash(Context& c) {
   c.hash_sorter.sort(c.hash_key.p, c.hash_val.p, nv, bits, c.stream, &skey, &sidx);
   cudaMemsetAsync(c.cell_start.p, 0xFF, sizeof(uint32_t) * table, c.stream);
   k_cell_bounds<<<grid_for(nv), kBlock, 0, c.stream>>>(skey, nv, c.cell_start.p, c.cell_end.p);
-  k_cache_neighbors<<<grid_for(nv), kBlock, 0, c.stream>>>(
-      sidx, c.cell_start.p, c.cell_end.p, c.x.p, c.x_init.p, nv, I,
-      (uint32_t)c.params.max_neighbor_size, c.neighbors.p);
+  // A lane's walk of its cells is a chain of about 100 us whatever the number of vertices; a warp per
+  // vertex has no chain but issues more.  11,495 vertices 102 -> 13 us with a warp, 65,536 108 -> 39,
+  // 4,096 33 -> 6, but 538,368 132 -> 162 and 917 k 372 -> 483: the line is where about 0.45 ns a vertex
+  // have grown to the chain.
+  if (nv <= 1600u * (uint32_t)c.num_sms)
+    k_cache_neighbors<<<grid_for(nv, kBlock / 32), kBlock, 0, c.stream>>>(
+        sidx, c.cell_start.p, c.cell_end.p, c.x.p, c.x_init.p, nv, I,
+        (uint32_t)c.params.max_neighbor_size, c.neighbors.p);
+  else
+    k_cache_neighbors_lane<<<grid_for(nv), kBlock, 0, c.stream>>>(
+        sidx, c.cell_start.p, c.cell_end.p, c.x.p, c.x_init.p, nv, I,
+        (uint32_t)c.params.max_neighbor_size, c.neighbors.p);
 }
 
 void launch_collide(Context& c, const FrameConst& k) {
