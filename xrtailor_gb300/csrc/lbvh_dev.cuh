@@ -190,7 +190,8 @@ __device__ __forceinline__ void write_node(const TreeMem& t, const int4& rec, f3
   }
 }
 
-// On through global memory from the subtree over [l, r], whose node is written.
+// On through global memory from the subtree over [l, r], whose node is written: by this thread, or
+// ahead of a barrier of the block.
 template <bool BUILD>
 __device__ __forceinline__ void tree_walk(const TreeMem& t, const int4& rec, TreeEnd l, TreeEnd r,
                                           f3 bl, f3 bu, uint32_t* err) {
@@ -203,7 +204,8 @@ __device__ __forceinline__ void tree_walk(const TreeMem& t, const int4& rec, Tre
     }
     const bool left = r.d > l.d;
     const uint32_t g = left ? r.pos : l.pos - 1;
-    // acq_rel: releases this subtree's box with its end; the second arrival acquires the first's
+    // acq_rel: releases this subtree's box with its end (the thread's own stores and those ordered
+    // before it by a barrier); the second arrival acquires the first's
     unsigned long long far;
     asm volatile("atom.acq_rel.gpu.global.exch.b64 %0, [%1], %2;"
                  : "=l"(far)
@@ -308,6 +310,9 @@ __device__ __forceinline__ void tree_up(const TreeMem& t, TreeShared& sh, uint32
           le.pos == i ? n - 1 + p : p, re.pos == i + 1 ? n + p : p + 1, le, re);
     }
   }
+  // A node is written by the thread at its split, its subtree carried on by another: the barrier
+  // orders all of the block's nodes before any of its exchanges, so that an exchange releases them.
+  __syncthreads();
   if (!valid || (waiting != kNone && sh.count[waiting] != 1u)) return;
   tree_walk<BUILD>(t, rec, l, r, bl, bu, err);
 }
