@@ -526,76 +526,83 @@ __global__ void k_query(LbvhView b, const float* __restrict__ q, uint32_t nq,
   counts[i] = found;
 }
 
-// A warp per query: the nodes still to be tested and the leaves that overlap are one list in the
-// order of the walk.  A round tests all its nodes and puts in the place of each what follows from
-// it: an overlapping leaf itself, below an overlapping inner node its left child, and after a left
-// child its sibling.  After about twice the depth of the tree only leaves are left, and the first
-// kMaxCandidates of them are the walk's.  A list that outgrows kFront is walked by one lane instead.
-constexpr uint32_t kFront = 512, kQueryBlock = 128;
-constexpr uint32_t kLeft = 1, kDone = 2;  // a left child; an overlapping leaf (its object)
-template <int KIND>
-__global__ void __launch_bounds__(kQueryBlock) k_query_warp(
+// G lanes per query (8 or 32).  What follows in the walk is a stack in shared memory, the next on top:
+// nodes to be tested and, behind one of those, leaves known to overlap.  A round takes up to G
+// entries, one a lane, and puts in the place of each what follows from it: an overlapping leaf
+// itself, below an overlapping inner node its left child, and after a left child its sibling.  The
+// leaves ahead of the first node left are the walk's next candidates and leave the stack; at
+// kMaxCandidates the walk ends.  A full round leaves kReserve entries free; without room for one,
+// entries are taken singly, which deepens the stack by at most one per level of the tree (64-bit
+// keys: 65 levels).
+constexpr uint32_t kQueryBlock = 128, kReserve = 72;
+// An entry: node, or object of a leaf, with its kind in the two top bits.
+constexpr uint32_t kLeft = 1u << 30, kDone = 2u << 30, kEntryIds = kLeft;
+template <int KIND, int G>
+__global__ void __launch_bounds__(kQueryBlock) k_query_group(
     LbvhView b, const float* __restrict__ q, uint32_t nq, uint32_t* __restrict__ counts,
     uint32_t* __restrict__ cands, uint32_t* err) {
-  constexpr unsigned kAll = 0xFFFFFFFFu;
-  __shared__ uint2 lists[kQueryBlock / 32][2][kFront];
-  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  constexpr unsigned kAll = 0xFFFFFFFFu, kGroup = G == 32 ? kAll : (1u << G % 32) - 1u;
+  constexpr uint32_t kStack = G == 32 ? 640 : 176;
+  static_assert(kReserve >= 65 + 2, "singly taken entries fit");
+  __shared__ uint32_t stacks[kQueryBlock / G][kStack];
+  const uint32_t lane = threadIdx.x % G, shift = (threadIdx.x & 31u) - lane;
   const unsigned below = (1u << lane) - 1u;
-  const uint32_t i = blockIdx.x * (kQueryBlock / 32) + wid;
-  if (i >= nq) return;
-  const TreeQuery<KIND> test(q, i);
+  const uint32_t i = blockIdx.x * (kQueryBlock / G) + threadIdx.x / G;
+  const bool valid = i < nq;
+  const TreeQuery<KIND> test(q, valid ? i : 0u);
   uint32_t* out = cands + (size_t)i * kMaxCandidates;
-  uint2 *cur = lists[wid][0], *next = lists[wid][1];
-  if (lane == 0) cur[0] = make_uint2(0u, 0u);
-  uint32_t count = b.n ? 1u : 0u;
-  bool open = count != 0, fits = true;
+  uint32_t* stack = stacks[threadIdx.x / G];
+  auto ballot = [&](bool p) { return __ballot_sync(kAll, p) >> shift & kGroup; };
+  if (lane == 0) stack[0] = 0u;  // the root
+  uint32_t count = valid && b.n ? 1u : 0u, found = 0;
   __syncwarp();
-  for (uint32_t round = 0; open && fits; ++round) {
-    if (round > 2 * b.n + 2) {
-      raise_error(err, kErrTraversal);
-      return;
+  for (uint32_t round = 0; __any_sync(kAll, count != 0); ++round) {
+    if (round > 2 * b.n + 2 || __any_sync(kAll, count > kStack - 2)) {
+      if (count != 0 && lane == 0) raise_error(err, kErrTraversal);
+      break;
     }
-    open = false;
-    uint32_t made = 0;
-    for (uint32_t base = 0; base < count && fits; base += 32) {
-      const uint2 e = base + lane < count ? cur[base + lane] : make_uint2(0u, 0u);
-      uint2 put[2];
-      uint32_t n = 0;
-      if (base + lane < count) {
-        if (e.y == kDone) {
-          put[n++] = e;
-        } else {
-          const float4 l = b.lo[e.x], h = b.hi[e.x];
-          if (test(l, h))
-            put[n++] = make_uint2((uint32_t)__float_as_int(l.w), e.x >= b.n - 1 ? kDone : kLeft);
-          if (e.y == kLeft) put[n++] = make_uint2((uint32_t)__float_as_int(h.w), 0u);
+    const uint32_t room = kStack - kReserve > count ? kStack - kReserve - count : 1u;
+    const uint32_t n = min(min(count, (uint32_t)G), room);
+    const uint32_t e = lane < n ? stack[count - 1 - lane] : 0u;
+    count -= n;
+    __syncwarp();
+    uint32_t first = 0, second = 0, made = 0;  // what follows from the entry, in order
+    if (lane < n) {
+      if (e & kDone) {
+        first = e;
+        made = 1;
+      } else {
+        const uint32_t node = e & (kEntryIds - 1);
+        const float4 l = b.lo[node], h = b.hi[node];
+        if (test(l, h)) {
+          first = (uint32_t)__float_as_int(l.w) | (node >= b.n - 1 ? kDone : kLeft);
+          made = 1;
+        }
+        if (e & kLeft) {
+          const uint32_t sibling = (uint32_t)__float_as_int(h.w);
+          if (made++) second = sibling;
+          else first = sibling;
         }
       }
-      const unsigned m1 = __ballot_sync(kAll, n & 1u), m2 = __ballot_sync(kAll, n & 2u);
-      const uint32_t at = made + __popc(m1 & below) + 2 * __popc(m2 & below);
-      made += __popc(m1) + 2 * __popc(m2);
-      fits = made <= kFront;
-      if (fits) {
-        if (n > 0) next[at] = put[0];
-        if (n > 1) next[at + 1] = put[1];
-      }
-      open = open || __any_sync(kAll, (n > 0 && put[0].y != kDone) || (n > 1 && put[1].y != kDone));
     }
+    const bool leaf = first & kDone;
+    const unsigned nodes = ballot(made > (leaf ? 1u : 0u));  // lanes with nodes left
+    // candidates: the leaves up to the first such lane's
+    const bool take = leaf && (nodes & below) == 0;
+    const unsigned taken = ballot(take);
+    const uint32_t at = found + __popc(taken & below);
+    if (take && at < kMaxCandidates) out[at] = first & (kEntryIds - 1);
+    found += __popc(taken);
+    const uint32_t keep = made - (take ? 1u : 0u);
+    const unsigned m1 = ballot(keep & 1u), m2 = ballot(keep & 2u);
+    uint32_t top = count + __popc(m1) + 2 * __popc(m2);  // one above the whole round's
+    count = found < kMaxCandidates ? top : 0u;
+    top -= __popc(m1 & below) + 2 * __popc(m2 & below);  // one above this lane's
+    if (keep > 0) stack[top - 1] = take ? second : first;
+    if (keep > 1) stack[top - 2] = second;
     __syncwarp();
-    uint2* t = cur;
-    cur = next;
-    next = t;
-    count = made;
   }
-  if (fits) {
-    count = min(count, kMaxCandidates);
-    for (uint32_t k = lane; k < count; k += 32) out[k] = cur[k].x;
-    if (lane == 0) counts[i] = count;
-  } else if (lane == 0) {
-    uint32_t found = 0;
-    lbvh_traverse(b, test, [&](uint32_t obj) { out[found++] = obj; }, err);
-    counts[i] = found;
-  }
+  if (valid && lane == 0) counts[i] = min(found, kMaxCandidates);
 }
 
 }  // namespace
@@ -751,14 +758,24 @@ void launch_refit_midstep(Lbvh& b, const float4* x1, const float4* n1, const int
   launch_refit(b, GrowMidstep{x1, n1, tri, tol, b.pred.p}, s, d_err);
 }
 
-// A lane's walk takes 260-300 us however few the queries (2.1 M triangles, about 10 leaves a box); a
-// warp's 49 us for 100 to 1,000 of them, 82 for 5,000, 209 for 20,000 and 723 for 80,000.
+// Lanes per query.  Few queries are bound by the chain of a walk (2.09 M triangles, boxes of about 29
+// leaves, 1,000 queries: one lane 73 us, 8 lanes 29, 32 lanes 21; of 256 and more leaves 240, 77 and
+// 35), many by issue: 6,000 queries that end near the root take 21, 20 and 28 us, 20,000 of them 24, 33
+// and 70 (but 20,000 of 29 leaves 112, 55 and 104).
+constexpr uint32_t kWarpQueries = 3000, kGroupQueries = 20000;
+template <int KIND, int G>
+static void launch_query_group(const Lbvh& b, const float* q, uint32_t nq, uint32_t* counts,
+                               uint32_t* cands, cudaStream_t s, uint32_t* err) {
+  k_query_group<KIND, G><<<grid_for(nq, kQueryBlock / G), kQueryBlock, 0, s>>>(b.view(), q, nq, counts,
+                                                                             cands, err);
+}
 template <int KIND>
 static void launch_query(const Lbvh& b, const float* q, uint32_t nq, uint32_t* counts,
                          uint32_t* cands, cudaStream_t s, uint32_t* err) {
-  if (nq <= 20000u)
-    k_query_warp<KIND><<<grid_for(nq, kQueryBlock / 32), kQueryBlock, 0, s>>>(b.view(), q, nq, counts,
-                                                                             cands, err);
+  if (nq <= kWarpQueries)
+    launch_query_group<KIND, 32>(b, q, nq, counts, cands, s, err);
+  else if (nq <= kGroupQueries)
+    launch_query_group<KIND, 8>(b, q, nq, counts, cands, s, err);
   else
     k_query<KIND><<<grid_for(nq), kBlock, 0, s>>>(b.view(), q, nq, counts, cands, err);
 }
