@@ -254,7 +254,8 @@ struct TiledSet {
   uint32_t max_step = 0;                // most constraints in one local color of one tile
   uint32_t block = 512;                 // threads per tile block (256 or 512)
   uint32_t block1 = 512;                // threads per block of the streamed kernels
-  uint32_t resident = 0;                // tile blocks the GPU holds at once (above: streamed)
+  uint32_t resident = 0;                // tile blocks with whole records the GPU holds at once
+  bool stream_more = false;             // ... and holds more of with streamed records
   std::vector<ColorRange> tile_colors;  // ranges of executed tiles per tile color
   std::vector<uint32_t> tile_color_cons;  // constraints per tile color (profiling units)
   DBuf<uint32_t> foot;                  // footprint vertices of every executed tile
@@ -657,7 +658,7 @@ size_t tile_smem_fwd(const TiledSet& T, bool stretch, bool whole);
 // float4 -> packed xyz (12 B per element) and back (w set to `w`), for host copies.
 void launch_pack_xyz(const float4* in, float* out, uint32_t n, cudaStream_t s);
 void launch_unpack_xyz(const float* in, float4* out, uint32_t n, float w, cudaStream_t s);
-// Sets T.block (256 / 512 threads) and T.resident; after configure_tile_kernels.
+// Sets T.block (256 / 512 threads), T.resident and T.stream_more; after configure_tile_kernels.
 cudaError_t choose_tile_block(TiledSet& T, bool bend);
 // tile-local Gauss-Seidel: all tiles of one tile color (range of executed tiles)
 // tape_x / tape_l (the adjoint's recorded replay): every projection's input positions (and

@@ -670,23 +670,30 @@ size_t tile_smem_fwd(const TiledSet& T, bool stretch, bool whole) {
 }
 
 // Block size of a tile set: 256 threads when the footprint fits 256 x kFootPerThread and a local
-// color's elements fill at most one pass, else 512; and how many of its blocks the GPU holds at once.
+// color's elements fill at most one pass, else 512; how many of its blocks the GPU holds at once, and
+// whether streamed records make that more.
 cudaError_t choose_tile_block(TiledSet& T, bool bend) {
   T.block = (T.max_foot <= 256u * kFootPerThread && T.max_step <= 256) ? 256 : 512;
   // streamed (throughput-regime) blocks: 256 threads whenever the footprint allows (a large color
   // takes a second pass, but twice the blocks fit on an SM)
   T.block1 = T.max_foot <= 256u * kFootPerThread ? 256 : T.block;
-  int dev = 0, sms = 0, per_sm = 0;
+  int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  const size_t smem = tile_smem_fwd(T, !bend, true);
-  const void* kern = bend ? (const void*)bend_tiles_kernel(T.block != 256, false, false)
-                          : (const void*)stretch_tiles_kernel(false, T.block != 256, false, false);
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)T.block, smem);
-  if (e != cudaSuccess) return e;
-  T.resident = (uint32_t)std::max(per_sm, 1) * (uint32_t)sms;
-  return cudaSuccess;
+  auto per_sm = [&](uint32_t block, bool stream) {
+    const void* kern = bend ? (const void*)bend_tiles_kernel(block != 256, stream, false)
+                            : (const void*)stretch_tiles_kernel(false, block != 256, stream, false);
+    int n = 0;
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)block,
+                                                        tile_smem_fwd(T, !bend, !stream));
+    return (uint32_t)std::max(n, 1);
+  };
+  const uint32_t whole = per_sm(T.block, false), streamed = per_sm(T.block1, true);
+  T.resident = whole * (uint32_t)sms;
+  T.stream_more = streamed > whole;
+  return e;
 }
 
 // float4 {x, y, z, w} <-> packed xyz, for the host copies of the C ABI (one DMA of 12 B per
@@ -725,12 +732,21 @@ void launch_unpack_xyz(const float* in, float4* out, uint32_t n, float w, cudaSt
 // 35.4 ms.
 static bool release_early(const TiledSet& T, uint32_t block) { return T.max_step <= block; }
 
+// Records stream in by local color when the launch has more tiles than fit at once and streaming
+// makes room for more of them; a tile whose whole block leaves as many resident only pays for the
+// streaming, a wait per color (300 cloths of 20 x 20 to 120 x 120, a bend launch of 64- / 128- /
+// 256-vertex tiles streamed 86 / 92 / 85 us, whole 58 / 67 / 68; a stretch launch 89 / 80 / 48 and
+// 72 / 64 / 40; 512-vertex bend tiles 57 and 50).
+static bool stream_records(const TiledSet& T, uint32_t nt) {
+  return nt > T.resident && T.stream_more;
+}
+
 void launch_stretch_tiles(Context& c, const FrameConst& k, ColorRange tiles, bool reset_lambda,
                           float4* tape_x, float* tape_l) {
   const uint32_t nt = tiles.end - tiles.begin;
   if (nt == 0) return;
   const TiledSet& T = c.s_tiles;
-  const bool stream = nt > T.resident;  // many waves of tiles: throughput regime
+  const bool stream = stream_records(T, nt);
   const uint32_t block = stream ? T.block1 : T.block;
   const uint32_t buf16 = stream ? 2 * T.max_seg16 : T.max_tile16;  // as tile_smem_fwd sizes it
   const StretchTilesK kern = stretch_tiles_kernel(reset_lambda, block != 256, stream, tape_x);
@@ -744,7 +760,7 @@ void launch_bend_tiles(Context& c, const FrameConst& k, ColorRange tiles, float4
   const uint32_t nt = tiles.end - tiles.begin;
   if (nt == 0) return;
   const TiledSet& T = c.b_tiles;
-  const bool stream = nt > T.resident;  // many waves of tiles: throughput regime
+  const bool stream = stream_records(T, nt);
   const uint32_t block = stream ? T.block1 : T.block;
   const BendTilesK kern = bend_tiles_kernel(block != 256, stream, tape_x);
   const uint32_t buf16 = stream ? 2 * T.max_seg16 : T.max_tile16;  // as tile_smem_fwd sizes it
