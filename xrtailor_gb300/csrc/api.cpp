@@ -1184,6 +1184,8 @@ xrt_status xrt_start(xrt_ctx* h) {
                         (int)c.h_ortri[f]);
     XRT_CUDA(&c, upload(c.otri, ot, c.stream));
     xrt::setup::build_vf(c.h_otri, c.onv, ptr, list);
+    for (size_t i = 0; i + 1 < ptr.size(); ++i)
+      c.longest_fan = std::max(c.longest_fan, ptr[i + 1] - ptr[i]);
     XRT_CUDA(&c, upload(c.ovf_ptr, ptr, c.stream));
     XRT_CUDA(&c, upload(c.ovf_list, list, c.stream));
     xrt::launch_vertex_normals(c.ox0.p, c.otri.p, c.ovf_ptr.p, c.ovf_list.p, c.on.p, c.onv, c.stream);

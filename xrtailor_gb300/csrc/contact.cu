@@ -28,11 +28,8 @@ __device__ __forceinline__ f3 lerp_pos(const float4* __restrict__ x0, const floa
 // The weighted sum of the face normals around each vertex of the warp, in list order.  The warp's
 // vertices own consecutive entries of the list: the lanes work out the terms of kFan entries at a
 // time, one entry a lane, whichever vertex owns it, and each vertex adds its own up from shared
-// memory.  A vertex has six faces as a rule, but a pole of a body of revolution its whole ring, and a
-// lane that takes its vertex's faces one after the other takes 27 us for a ring of 84.
-// 6,890 vertices with such poles: 29 -> 9.4 us, 165,360 of them 44 -> 22 us; without poles 4,096 vertices
-// take 9.8 us against 7.7 and 642 take 8.1 against 7.5 (the owner's position is read once more per
-// face).
+// memory.  A vertex has six faces as a rule, but a pole of a body of revolution its whole ring, which
+// would be one lane's chain.
 constexpr int kFanBlock = 64;
 constexpr uint32_t kFanRounds = 6, kFan = 32 * kFanRounds;
 struct FanShared {
@@ -88,14 +85,48 @@ __device__ __forceinline__ f3 fan_sum(FanShared& w, const int4* __restrict__ tri
   return acc;
 }
 
-__global__ void __launch_bounds__(kFanBlock) k_obstacle_pass(
+// The same with a lane that takes its vertex's faces one after the other, every position once.
+template <class Pos>
+__device__ __forceinline__ f3 fan_walk(const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
+                                       const uint32_t* __restrict__ list, uint32_t i, uint32_t nv,
+                                       Pos pos) {
+  f3 acc = mk3(0, 0, 0);
+  if (i >= nv) return acc;
+  const f3 xi = pos((int)i);
+  for (uint32_t k = ptr[i]; k < ptr[i + 1]; ++k) {
+    const uint32_t fc = list[k];
+    const int4 t = tri[fc >> 2];
+    const uint32_t j = fc & 3u;
+    const f3 a = pos(j == 0 ? t.y : j == 1 ? t.z : t.x) - xi;
+    const f3 b = pos(j == 0 ? t.z : j == 1 ? t.x : t.y) - xi;
+    acc = acc + cross(a, b) / (dot(a, a) * dot(b, b));
+  }
+  return acc;
+}
+
+// SPREAD: fan_sum, else fan_walk (uses_spread_fans).
+template <bool SPREAD>
+constexpr int kFanThreads = SPREAD ? kFanBlock : kBlock;
+template <bool SPREAD, class Pos>
+__device__ __forceinline__ f3 fan(const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
+                                  const uint32_t* __restrict__ list, uint32_t i, uint32_t nv,
+                                  Pos pos) {
+  if constexpr (SPREAD) {
+    __shared__ FanShared shared[kFanBlock / 32];
+    return fan_sum(shared[threadIdx.x >> 5], tri, ptr, list, i, nv, pos);
+  } else {
+    return fan_walk(tri, ptr, list, i, nv, pos);
+  }
+}
+
+template <bool SPREAD>
+__global__ void __launch_bounds__(kFanThreads<SPREAD>) k_obstacle_pass(
     const float4* __restrict__ x0, const float4* __restrict__ x, float4* __restrict__ x1,
     float4* __restrict__ n1, const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
     const uint32_t* __restrict__ list, uint32_t nv, float alpha) {
-  __shared__ FanShared shared[kFanBlock / 32];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const f3 acc = fan_sum(shared[threadIdx.x >> 5], tri, ptr, list, i, nv,
-                         [&](int j) { return lerp_pos(x0, x, j, alpha); });
+  const f3 acc =
+      fan<SPREAD>(tri, ptr, list, i, nv, [&](int j) { return lerp_pos(x0, x, j, alpha); });
   if (i >= nv) return;
   x1[i] = mk4(lerp_pos(x0, x, i, alpha), 0.0f);
   n1[i] = mk4(normalize(acc), 0.0f);
@@ -104,22 +135,19 @@ __global__ void __launch_bounds__(kFanBlock) k_obstacle_pass(
 __global__ void __launch_bounds__(kFanBlock) k_vertex_normals(
     const float4* __restrict__ x, const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
     const uint32_t* __restrict__ list, float4* __restrict__ out, uint32_t nv) {
-  __shared__ FanShared shared[kFanBlock / 32];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const f3 acc = fan_sum(shared[threadIdx.x >> 5], tri, ptr, list, i, nv,
-                         [&](int j) { return mk3(x[j]); });
+  const f3 acc = fan<true>(tri, ptr, list, i, nv, [&](int j) { return mk3(x[j]); });
   if (i < nv) out[i] = mk4(normalize(acc), 0.0f);
 }
 
 // Frame end: x0 = x, then normals of the new x0 (computed from x, which is the same data).
-__global__ void __launch_bounds__(kFanBlock) k_obstacle_commit(
+template <bool SPREAD>
+__global__ void __launch_bounds__(kFanThreads<SPREAD>) k_obstacle_commit(
     const float4* __restrict__ x, float4* __restrict__ x0, float4* __restrict__ nrm,
     const int4* __restrict__ tri, const uint32_t* __restrict__ ptr,
     const uint32_t* __restrict__ list, uint32_t nv) {
-  __shared__ FanShared shared[kFanBlock / 32];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const f3 acc = fan_sum(shared[threadIdx.x >> 5], tri, ptr, list, i, nv,
-                         [&](int j) { return mk3(x[j]); });
+  const f3 acc = fan<SPREAD>(tri, ptr, list, i, nv, [&](int j) { return mk3(x[j]); });
   if (i >= nv) return;
   x0[i] = mk4(mk3(x[i]), 0.0f);
   nrm[i] = mk4(normalize(acc), 0.0f);
@@ -528,12 +556,24 @@ __global__ void __launch_bounds__(kGenBlock) k_generate_ee(LbvhForest F, InstVie
 
 }  // namespace
 
+// One wave of spread blocks (512 vertices an SM) is faster for bodies of revolution whatever the ring
+// (ring 84, 6,890 vertices 30 -> 5.6 us) and up to 1.5 us either way for meshes without poles.  Beyond it
+// a lane per vertex is, until its longest ring, 0.32 us a face, takes longer than the extra waves:
+// without poles 78,400 vertices take 12.0 us spread and 7.2 a lane each, 160,000 19.9 and 10.1; ring 24
+// 82,680 10.0 and 11.8, 165,000 15.8 and 13.0; ring 48 165,000 17.3 and 27.5, 330,000 33.6 and 32.3; ring
+// 84 660,000 62 and 70, 1.4 M 119 and 91.
+static bool uses_spread_fans(const Context& c) {
+  return c.onv <= 512u * (uint32_t)c.num_sms || c.longest_fan > c.onv / 5000u;
+}
+
 void launch_obstacle_pass(Context& c, int step, int num_steps) {
   if (c.onv == 0) return;
   const float alpha = ((float)step + 1.0f) / (float)num_steps;
-  k_obstacle_pass<<<grid_for(c.onv, kFanBlock), kFanBlock, 0, c.stream>>>(c.ox0.p, c.ox.p, c.ox1.p, c.on1.p,
-                                                            c.otri.p, c.ovf_ptr.p, c.ovf_list.p,
-                                                            c.onv, alpha);
+  const bool spread = uses_spread_fans(c);
+  const unsigned block = spread ? kFanThreads<true> : kFanThreads<false>;
+  (spread ? k_obstacle_pass<true> : k_obstacle_pass<false>)<<<grid_for(c.onv, block), block, 0,
+                                                               c.stream>>>(
+      c.ox0.p, c.ox.p, c.ox1.p, c.on1.p, c.otri.p, c.ovf_ptr.p, c.ovf_list.p, c.onv, alpha);
   launch_refit_midstep(c.bvh, c.ox1.p, c.on1.p, c.otri.p, c.params.bvh_tolerance, c.stream, c.err.p);
 }
 
@@ -572,8 +612,11 @@ void launch_generate_contacts(Context& c) {
 
 void launch_obstacle_commit(Context& c) {
   if (c.onv == 0) return;
-  k_obstacle_commit<<<grid_for(c.onv, kFanBlock), kFanBlock, 0, c.stream>>>(c.ox.p, c.ox0.p, c.on.p, c.otri.p,
-                                                              c.ovf_ptr.p, c.ovf_list.p, c.onv);
+  const bool spread = uses_spread_fans(c);
+  const unsigned block = spread ? kFanThreads<true> : kFanThreads<false>;
+  (spread ? k_obstacle_commit<true> : k_obstacle_commit<false>)<<<grid_for(c.onv, block), block, 0,
+                                                                   c.stream>>>(
+      c.ox.p, c.ox0.p, c.on.p, c.otri.p, c.ovf_ptr.p, c.ovf_list.p, c.onv);
 }
 
 void launch_vertex_normals(const float4* x, const int4* tri, const uint32_t* ptr,

@@ -519,6 +519,7 @@ struct Context {
   DBuf<float4> ox0, ox, ox1, on, on1;
   DBuf<int4> otri;                   // a, b, c, r-triangle mask
   DBuf<uint32_t> ovf_ptr, ovf_list;
+  uint32_t longest_fan = 0;          // most faces around one obstacle vertex
   Lbvh bvh;
   ProximityState prox;
   ImpactZoneState izone;
