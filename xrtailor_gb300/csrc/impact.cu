@@ -362,6 +362,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kZT * G)
       __stcg(&a.lambda[eb + e], tmin(__ldcg(&a.lambda[eb + e]) + kMu * c, 0.0f));
     }
   }
+  zone_sync<C>(cl);  // block 0 does not leave while others read its shared memory
   if (tid == 0 && rank == 0) a.conv[zi] = conv_it;
 }
 
