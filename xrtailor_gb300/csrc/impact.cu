@@ -1002,15 +1002,17 @@ xrt_status solve_zones(Context& c, const Graph& g, float obstacle_mass, float th
   const uint32_t n0 = off[1], n1 = off[2] - off[1], n2 = off[3] - off[2], n3 = off[4] - off[3];
   by_group[0] += n2;
   by_group[1] += n3;
-  // a launch whose zones all have at most one element per thread keeps them in registers
+  // a launch whose zones all have at most one element per thread keeps them in registers; beyond are
+  // zones of more than 16,384 elements, or of more than 8 (16) chunks where the device does not hold
+  // the wider clusters
   const uint32_t widest[4] = {kZT, kZoneCluster * kZT, kZoneClusterWide * kZT,
                               kZoneClusterWide * kWideGroups * kZT};
-  bool one[4] = {true, true, true, true};
-  for (int g = 0; g < 4; ++g)
+  bool one[4] = {true, true, true, true};  // one[0] by its group
+  for (int g = 1; g < 4; ++g)
     for (int32_t q : group[g])
       one[g] &= (uint32_t)std::max(zone[q].y - zone[q].x, zone[q].w - zone[q].z) <= widest[g];
   const int32_t* ids = z.zid.p;
-  if (n0) (one[0] ? k_zone_solve_one<1, 1> : k_zone_solve<1, 1>)<<<n0, kZT, 0, s>>>(a, ids);
+  if (n0) k_zone_solve_one<1, 1><<<n0, kZT, 0, s>>>(a, ids);
   if (n1)
     (one[1] ? k_zone_solve_one<kZoneCluster, 1> : k_zone_solve<kZoneCluster, 1>)
         <<<n1 * kZoneCluster, kZT, 0, s>>>(a, ids + off[1]);
