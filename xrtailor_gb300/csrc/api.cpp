@@ -1736,7 +1736,7 @@ xrt_status xrt_lbvh_build_device(xrt_lbvh* b, const float* d_prims, const float*
   if (!b || (n && !d_prims)) return XRT_ERR_INVALID_ARGUMENT;
   cudaSetDevice(b->device);
   cudaStream_t s = stream ? (cudaStream_t)stream : b->stream;
-  if (b->b.reserve(n) != cudaSuccess) return XRT_ERR_CUDA;
+  if (b->b.reserve(n, /*packed=*/true) != cudaSuccess) return XRT_ERR_CUDA;
   b->b.n = n;
   b->b.construct(scr, s, b->err.p, d_prims, d_pred ? d_pred : d_prims);
   return cudaGetLastError() == cudaSuccess ? XRT_OK : XRT_ERR_CUDA;

@@ -86,7 +86,7 @@ struct LbvhView {
 
 // A forest of independent trees over consecutive primitive ranges (segments), in shared arrays.
 // Segment s owns primitives [prim_base, prim_base + n), nodes [node_base, node_base + 2n - 1)
-// (internal nodes first, then leaves, as in a single tree) and merge counters
+// (internal nodes first, then leaves, as in a single tree) and the exported escapes of internal nodes
 // [internal_base, internal_base + n - 1).  Every link is local to its segment, so each segment is
 // bit for bit the tree its primitives alone would give.  One segment = the classic single tree.
 struct LbvhForest {
@@ -101,7 +101,7 @@ struct Lbvh {
   uint32_t nodes = 0;              // total nodes (sum of 2 n_s - 1 over non-empty segments)
   uint32_t internal = 0;           // total internal nodes
   bool active = false;
-  DBuf<float4> v, pred;            // 3 per primitive
+  DBuf<float4> v, pred;            // 3 per primitive (none in a packed tree)
   DBuf<float4> leaf_lo, leaf_hi;   // per primitive (original order) before sorting
   DBuf<float4> lo, hi;             // per node
   DBuf<int4> node;                 // parent, left, right, object (segment-local)
@@ -130,7 +130,8 @@ struct Lbvh {
   // Segments of the forest: primitive counts in primitive order (empty = one segment).
   // Uploads the table; call before reserve.
   cudaError_t set_segments(const std::vector<uint32_t>& counts, cudaStream_t s);
-  cudaError_t reserve(uint32_t n_prims);
+  // `packed`: a tree that is only built from 9 floats per primitive, without v and pred.
+  cudaError_t reserve(uint32_t n_prims, bool packed = false);
   // BVH::Construct(scr) on v / pred already in device memory (BVH.cu:618-722), every segment; or on
   // 9 floats per primitive (single trees; p9 = pred).
   void construct(float scr, cudaStream_t s, uint32_t* d_err, const float* v9 = nullptr,

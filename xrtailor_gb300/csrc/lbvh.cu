@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kBlock) k_leaf_boxes(Prims P, uint32_t n, floa
   __shared__ uint32_t s_ext[6], s_seg;
   const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
   Box b = empty_box();
-  const uint32_t seg = i < n ? forest_find(F, i, 0) : 0xFFFFFFFFu;
+  const uint32_t seg = i < n ? forest_find(F, i) : 0xFFFFFFFFu;
   if (threadIdx.x < 6) s_ext[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_seg = seg;
   if (i < n) {
@@ -174,7 +174,7 @@ __global__ void k_morton(const float4* __restrict__ leaf_lo, const float4* __res
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   morton[i] = morton_of(Box{mk3(leaf_lo[i]), mk3(leaf_hi[i])},
-                        root_all + 6 * (size_t)forest_find(F, i, 0));
+                        root_all + 6 * (size_t)forest_find(F, i));
   index[i] = i;
 }
 
@@ -184,7 +184,7 @@ __global__ void k_seg_keys(const uint32_t* __restrict__ sindex, uint32_t n, uint
                            uint32_t* __restrict__ val, LbvhForest F) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  key[i] = forest_find(F, sindex[i], 0);
+  key[i] = forest_find(F, sindex[i]);
   val[i] = i;
 }
 __global__ void k_seg_gather(const uint32_t* __restrict__ perm, const uint32_t* __restrict__ m_in,
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kBlock) k_deltas(const uint32_t* __restrict__ 
   const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
   bool same = false;
   if (i < n) {
-    const int4 r = forest_rec(F, forest_find(F, i, 0));
+    const int4 r = forest_rec(F, forest_find(F, i));
     uint8_t d = 0;
     if (i + 1 < (uint32_t)(r.x + r.y)) {
       const uint32_t m0 = smorton[i], m1 = smorton[i + 1];
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kTreeBlock) k_tree(const uint32_t* __restrict_
     obj = sindex[i];
     bl = mk3(leaf_lo[obj]);
     bu = mk3(leaf_hi[obj]);
-    obj -= (uint32_t)forest_rec(t.F, forest_find(t.F, i, 0)).x;
+    obj -= (uint32_t)forest_rec(t.F, forest_find(t.F, i)).x;
   }
   if (SMALL)
     small_tree<true>(t, *reinterpret_cast<SmallShared*>(smem), i, i < n, obj, bl, bu, err);
@@ -623,15 +623,17 @@ cudaError_t Lbvh::set_segments(const std::vector<uint32_t>& counts, cudaStream_t
   return e;
 }
 
-cudaError_t Lbvh::reserve(uint32_t np) {
+cudaError_t Lbvh::reserve(uint32_t np, bool packed) {
   const size_t nn = np ? 2 * (size_t)np - 1 : 1;
   cudaError_t e = cudaSuccess;
   if (nseg() > 1) {
     if (e == cudaSuccess) e = skey.reserve(np);
     if (e == cudaSuccess) e = sval.reserve(np);
   }
-  if (e == cudaSuccess) e = v.reserve(3 * (size_t)np);
-  if (e == cudaSuccess) e = pred.reserve(3 * (size_t)np);
+  if (!packed) {
+    if (e == cudaSuccess) e = v.reserve(3 * (size_t)np);
+    if (e == cudaSuccess) e = pred.reserve(3 * (size_t)np);
+  }
   if (e == cudaSuccess) e = leaf_lo.reserve(np);
   if (e == cudaSuccess) e = leaf_hi.reserve(np);
   if (e == cudaSuccess) e = lo.reserve(nn);

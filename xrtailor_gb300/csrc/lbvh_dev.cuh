@@ -65,26 +65,17 @@ __device__ __forceinline__ int4 forest_rec(const LbvhForest& F, uint32_t s) {
   return F.nseg == 1 ? F.one : F.seg[s];
 }
 
-// Segment owning element i of a forest-wide range: field 0 = primitive / sorted leaf position,
-// 2 = node, 3 = internal node.  The last segment whose base is <= i: empty segments share their
-// base with the next one, so the segment found always owns i.
-__device__ __forceinline__ uint32_t forest_find(const LbvhForest& F, uint32_t i, int field) {
+// Segment owning primitive / sorted leaf position i.  The last segment whose base is <= i: empty
+// segments share their base with the next one, so the segment found always owns i.
+__device__ __forceinline__ uint32_t forest_find(const LbvhForest& F, uint32_t i) {
   if (F.nseg == 1) return 0;
   uint32_t lo = 0, hi = F.nseg;  // base(lo) <= i < base(hi)
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
-    const int4 r = F.seg[mid];
-    const uint32_t b = (uint32_t)(field == 0 ? r.x : (field == 2 ? r.z : r.w));
-    if (b <= i) lo = mid;
+    if ((uint32_t)F.seg[mid].x <= i) lo = mid;
     else hi = mid;
   }
   return lo;
-}
-
-// The tree of segment s with local links; objects are local, global = rec.x + object.
-__device__ __forceinline__ LbvhView forest_view(const LbvhForest& F, uint32_t s) {
-  const int4 r = forest_rec(F, s);
-  return LbvhView{(uint32_t)r.y, F.all.pred + 3 * (size_t)r.x, F.all.lo + r.z, F.all.hi + r.z};
 }
 
 // ---- bottom-up merge (AssignAABBCAS_Kernel, BVH.cu:515-538) -------------------------------------
@@ -241,7 +232,7 @@ __device__ __forceinline__ void tree_up(const TreeMem& t, TreeShared& sh, uint32
   sh.count[threadIdx.x] = 0;
   __syncthreads();
   const uint32_t c0 = i - threadIdx.x;  // the block's first position
-  const int4 rec = valid ? forest_rec(t.F, forest_find(t.F, i, 0)) : make_int4(0, 0, 0, 0);
+  const int4 rec = valid ? forest_rec(t.F, forest_find(t.F, i)) : make_int4(0, 0, 0, 0);
   const uint32_t base = (uint32_t)rec.x, n = (uint32_t)rec.y;
   TreeEnd l{i, 0, 0}, r{i, 0, 0};
   if (valid) {
@@ -526,7 +517,7 @@ __global__ void __launch_bounds__(kTreeBlock) k_refit(uint32_t n, Grow grow, Tre
   uint32_t obj = 0;
   f3 bl = mk3(0, 0, 0), bu = bl;
   if (i < n) {
-    const int4 r = forest_rec(t.F, forest_find(t.F, i, 0));
+    const int4 r = forest_rec(t.F, forest_find(t.F, i));
     const uint32_t k = (uint32_t)r.z + (uint32_t)r.y - 1 + (i - (uint32_t)r.x);
     const float4 l = t.lo[k], h = t.hi[k];
     obj = (uint32_t)__float_as_int(l.w);
