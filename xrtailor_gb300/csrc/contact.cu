@@ -221,7 +221,7 @@ __device__ __forceinline__ void keep_nearest(unsigned long long& key, float dist
 
 struct PairStack {
   uint2 e[kStack];      // node of the query's tree; query | left child << 5 | mask << 6
-  int4 tree[32];        // of each query: first node, primitives, first primitive
+  int4 tree[32];        // of each query's tree: first primitive, primitives, first node
 };
 // Takes packets of `packet` queries until none of `nq` is left.  start(i) sets the lane's query up
 // and returns its mask of tests (0: none) and its tree's record; within(slot, mask) leaves the tests

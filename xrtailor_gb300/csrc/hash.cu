@@ -460,9 +460,9 @@ void launch_hash(Context& c) {
   cudaMemsetAsync(c.cell_start.p, 0xFF, sizeof(uint32_t) * table, c.stream);
   k_cell_bounds<<<grid_for(nv), kBlock, 0, c.stream>>>(skey, nv, c.cell_start.p, c.cell_end.p);
   // A lane's walk of its cells is a chain of about 100 us whatever the number of vertices; a warp per
-  // vertex has no chain but issues more.  11,495 vertices 102 -> 13 us with a warp, 65,536 108 -> 39,
-  // 4,096 33 -> 6, but 538,368 132 -> 162 and 917 k 372 -> 483: the line is where about 0.45 ns a vertex
-  // have grown to the chain.
+  // vertex has no chain but issues more: 65,536 vertices 108 us by lanes and 39 by warps, 917 k 372 and
+  // 483.  A hash's kernels take 11.6 and 10.7 us on average at 193,600 vertices, 12.5 and 12.4 at 243,049,
+  // 12.9 and 13.2 at 270,400, 18.5 and 20.3 at 490,000.
   if (nv <= 1600u * (uint32_t)c.num_sms)
     k_cache_neighbors<<<grid_for(nv, kBlock / 32), kBlock, 0, c.stream>>>(
         sidx, c.cell_start.p, c.cell_end.p, c.x.p, c.x_init.p, nv, I,
@@ -475,11 +475,10 @@ void launch_hash(Context& c) {
 
 void launch_collide(Context& c, const FrameConst& k) {
   const uint32_t block = c.vertex_block;
-  // Four lanes per vertex for at most two and a half waves of them: a list's round trips and terms
-  // side by side shorten the launch (65,536 vertices 10.7 -> 8.8 us, the garment's frame 12.1 -> 11.2
-  // ms against 12.5 with the queue); with more vertices the instructions count, and the queue issues
-  // half as many (917 k vertices of 24 garments 118 -> 68 us against 118 with four lanes).  160,000
-  // vertices are the first measured size where the queue's frame is shorter (9.76 against 9.95 ms).
+  // Four lanes per vertex shorten a launch that is bound by its lists' round trips; with many vertices
+  // the instructions count, of which the queue issues half as many.  Frames of a folded sheet, four
+  // lanes and queue: 65,536 vertices 2.18 and 2.25 ms, 108,900 2.82 and 2.83, 129,600 3.02 and 3.00,
+  // 160,000 3.41 and 3.34; a launch on 917 k vertices 118 and 68 us.
   if (c.nv > 720u * (uint32_t)c.num_sms) {
     const size_t smem = sizeof(CollideShared) * (block / 32);
     if (raise_smem((const void*)k_collide_queue, smem) != cudaSuccess) return;

@@ -197,7 +197,7 @@ __device__ __forceinline__ void zone_sync(cg::cluster_group& cl) {
   }
 }
 
-// One zone per cluster of C blocks (C = 1 for zones of at most 256 nodes and impacts).  Block r
+// One zone per cluster of C blocks, of any number of chunks.  Block r
 // of the cluster owns the 256-element chunks ch = r, r + C, ...: it computes their values and
 // chunk sums and writes the sums into block 0's shared memory (distributed shared memory); after
 // a cluster barrier every block reads the chunk sums from block 0 and sums them by the same

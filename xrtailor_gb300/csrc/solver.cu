@@ -118,9 +118,9 @@ __global__ void k_stretch(const int4* __restrict__ con, float* __restrict__ lamb
 // 768 x 701 sheet 11.4 -> 9.1 ms.  NT threads per block: 512 for footprints up to
 // 4,096 vertices, 256 (twice the resident blocks per SM) up to 2,048.
 // Stretch tiles: the record block holds one segment per local color, as for bend (16-bit ids,
-// then float2 rest length and stretch_alpha(compliance, dt), each padded to 16 bytes).  STREAM (throughput regime):
-// the segments stream in two colors ahead through two shared-memory buffers; otherwise the whole
-// block comes in one bulk copy.  The multipliers of the tile's constraints stay in shared memory
+// then float2 rest length and stretch_alpha(compliance, dt), each padded to 16 bytes).  STREAM
+// (stream_records): the segments stream in two colors ahead through two shared-memory buffers;
+// otherwise the whole block comes in one bulk copy.  The multipliers of the tile's constraints stay in shared memory
 // from the prologue to the write-back.
 template <bool RESET, int NT, bool STREAM, bool TAPE>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_stretch_tiles(
@@ -399,9 +399,7 @@ struct TailArgs {
 
 // LRA + VF, per vertex.  AHEAD: the slots' lists (setup-time) are read ahead of the wait, and their
 // positions in one round with the vertex's own and the contacts' triangles; a second round brings
-// the contacts, with the normals their generation stored (computed here from the triangle's
-// corners before: 6.0 -> 5.2 us at 65,536 vertices, two slots).  At 917 k vertices AHEAD is 18.2 us
-// against 17.0 without.
+// the contacts, with the normals their generation stored.
 template <bool LRA, bool CONTACTS, bool TAPE, bool AHEAD>
 __global__ void k_stage(const TailArgs a) {
   pdl_release();
@@ -808,7 +806,10 @@ static TailArgs tail_args(Context& c, const FrameConst& k) {
   return a;
 }
 
-// Lists ahead of the wait while all vertices are in flight at once.
+// Lists ahead of the wait are for launches bound by their round trips.  A frame of a draped sheet with
+// two slots takes 2.20 ms without and 2.18 with them at 65,536 vertices; a launch 7.6 and 7.8 us at 97,344,
+// 9.6 and 9.6 at 202,500, 13.7 and 15.4 at 490,000 (their registers cost more than the round trip):
+// between, either form is within 0.5 us.
 template <bool TAPE, bool AHEAD>
 static void stage(Context& c, const TailArgs& a, bool lra, bool contacts) {
   auto kern = lra ? (contacts ? k_stage<true, true, TAPE, AHEAD> : k_stage<true, false, TAPE, AHEAD>)
