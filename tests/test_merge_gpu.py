@@ -71,3 +71,24 @@ def test_forest_rounds_match_single_trees(xrt):
             np.testing.assert_array_equal(bits(f["aabbs"][node:node + m]), bits(t["aabbs"]))
             node += m
         assert node == len(f["aabbs"])
+
+
+def test_ccd_refit_rounds_match_oracle(xrt):
+    """The obstacle's boxes grow by its motion, refit after refit, each further out than the one before."""
+    from tests.helpers import make_pair
+    from xrtailor_gb300 import scenes
+    body = scenes.icosphere(5, 0.3, center=(0.5, 0.0, 0.5))  # 20,480 triangles
+    cloth = scenes.grid_cloth(4, 1.0, origin=(0.0, 3.0, 0.0), jitter=1e-3, seed=1)
+    p = scenes._params(num_substeps=1, num_iterations=1, num_collision_passes=1, solve_bending=0,
+                       enable_self_collision=0)
+    g, o = make_pair(p, [cloth], [body])
+    rng = np.random.default_rng(3)
+    for k in range(8):
+        far = rng.normal(0, 5.0 * (k + 1), 3).astype(np.float32)
+        target = (body.positions * np.float32(1 + k) + far).astype(np.float32)
+        for s in (g, o):
+            s.set_obstacle_targets(target)
+            s.obstacle_bvh_update_ccd()
+        a, b = g.export_obstacle_bvh(), o.export_obstacle_bvh()
+        np.testing.assert_array_equal(a["nodes"], b["nodes"])
+        np.testing.assert_array_equal(bits(a["aabbs"]), bits(b["aabbs"]))
